@@ -35,10 +35,11 @@ __host__ __device__ inline EighSmemLayout eigh_smem_layout(int n, int nR, int nt
   return L;
 }
 
-// doubles of global scratch per CTA
+// doubles of global scratch per CTA: an even number, as the slots hold double2 arrays
+// (an odd order's 3 n^2 would put every other CTA's reflectors off their 16-byte alignment)
 __host__ __device__ inline int64_t eigh_slot_doubles(int n, int a_in_smem, bool need_uwork) {
   const int64_t nn = (int64_t)n * n;
-  if (a_in_smem) return 3 * nn;                  // R (2nn) | Qs
+  if (a_in_smem) return (3 * nn + 1) / 2 * 2;    // R (2nn) | Qs
   return 4 * nn + (need_uwork ? 2 * nn : 0);     // A (2nn) | Q | Qt | U work
 }
 
