@@ -63,6 +63,9 @@ const char* lqm_last_error(const lqm_ctx* ctx);
 int lqm_ctx_set_timeout(lqm_ctx* ctx, double seconds);
 /* Eigensolver path selection: orders n >= n_min use the batched blocked path
  * (panel reduction + batched GEMMs); 0 (default) selects it from n = 224 on.
+ * Below it the staged path (one kernel per stage for a whole list of k-points)
+ * serves orders up to 144 and the one-CTA kernel the others; a non-zero n_min
+ * holds every order below it to the one-CTA kernel.
  * No reference counterpart (the reference always calls LAPACK zheevr). */
 int lqm_ctx_set_blocked_min_n(lqm_ctx* ctx, int64_t n_min);
 /* Reduction of the blocked path: 1 two-stage (dense -> band of half-bandwidth 16 by
@@ -108,8 +111,9 @@ int lqm_ctx_set_scf_terms(lqm_ctx* ctx, int hartree, int fock);
 int lqm_ctx_set_scf_exchange(lqm_ctx* ctx, int64_t ns, int64_t nJ, int32_t d, const int64_t* jkeys,
                              const double* jblocks, int64_t n, const int64_t* siteof, const int64_t* flavorof);
 int lqm_ctx_scf_exchange_energy(const lqm_ctx* ctx, double* eJ);
-/* Block size (threads, a multiple of 32 up to 512; 0 restores the built-in rule)
- * of the one-CTA eigensolver for order n on this context.  No reference
+/* Block size (threads, a multiple of 32 up to 512) of the one-CTA eigensolver for
+ * order n on this context, which then serves that order; 0 restores the built-in
+ * rule, under which orders up to 144 take the staged path instead.  No reference
  * counterpart (a device launch parameter). */
 int lqm_ctx_set_eigh_threads(lqm_ctx* ctx, int64_t n, int nt);
 /* Autotuner of that block size for H's order (below the blocked path): every
@@ -117,7 +121,8 @@ int lqm_ctx_set_eigh_threads(lqm_ctx* ctx, int64_t n, int nt);
  * built-in rule's size up to four times it, or 512, whose shared-memory plan
  * fits) runs the eigen pass on the nk sample k-points (rho_k at mu = 0, T = 0.01
  * when want_rho, else eigenvectors), warmed up once and timed once with CUDA
- * events; the fastest becomes the context's block size for n (the sample should
+ * events; the fastest becomes the context's block size for n, and n keeps the staged
+ * path where that is faster than all of them (the sample should
  * span several waves of CTAs, e.g. the production k-grid, or it times latency
  * rather than throughput).  best_nt/best_ms
  * receive the choice, cand_nt/cand_ms (up to ncand_max, may be NULL) every
@@ -274,12 +279,13 @@ int lqm_bands_dos_rho_dev(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const dou
                           int precision);
 
 /* lqm_bands_dos_rho_dev for several models of uneven order on the same k list, with
- * ONE eigensolver launch for all of them: the batched form of the per-model loop of
+ * one eigen pass for all of them: the batched form of the per-model loop of
  * `bandmatrix` / `getdos` / `getdensitymatrix!` (src/modules/Spectrum/bands.jl:164-204,
  * dos.jl:202-223, densitymatrix.jl:28-49), which the reference runs model by model.
- * Each model's k-points go to CTA sub-teams of that model's one-CTA block size
- * (several teams per CTA on named barriers), so small orders fill the SMs as large
- * ones drain.  Models: 1..4, all below the blocked eigensolver's switch; arrays of
+ * Orders of the staged path run there, model after model.  Where one of them is held to
+ * the one-CTA kernel, all are ONE launch of it: each model's k-points go to CTA sub-teams
+ * of that model's block size (several teams per CTA on named barriers), so small orders
+ * fill the SMs as large ones drain.  Models: 1..4, all below the blocked eigensolver's switch; arrays of
  * nmodels entries (H, nL, Lkeys, d_rho, d_omegas, d_dos, d_bands; eband receives
  * nmodels values); d_w NULL means 1/nk. */
 int lqm_bands_dos_rho_multi_dev(lqm_ctx* ctx, int nmodels, const lqm_hops* const* H, int64_t nk,

@@ -23,6 +23,7 @@
 #include "kspace.h"
 #include "lqm_kernels.cuh"
 #include "lqm_large.cuh"
+#include "lqm_staged.cuh"
 #include "lqm_hf.cuh"
 #include "lqm_zgemm.cuh"
 #include "lqm_plan.h"
@@ -58,8 +59,9 @@ struct lqm_ctx {
   int num_sms = 0;
   double last_ms = 0.0;
   std::map<int, PlanDev> plans;
-  std::map<int, int> eigh_nt;  // one-CTA eigensolver block size per order n (autotuned or set), else the rule
-  DevBuf ws[52];
+  std::map<int, int> eigh_nt;     // one-CTA eigensolver block size per order n where that kernel was chosen (set or autotuned)
+  std::map<int, int> eigh_nt_alt; // autotuned block size where the staged path was faster (the kernel's other uses)
+  DevBuf ws[64];
   // per-kernel device-time statistics (CUDA events on the context stream)
   bool stats_on = false;
   bool phases_on = false;  // per-phase cycle counters inside the eigensolver (clock reads)
@@ -267,9 +269,10 @@ bool hops_buffer_keep(lqm_ctx* ctx, void* p, size_t bytes) {
 enum WsSlot {
   WS_SCRATCH = 0, WS_KS, WS_BANDS, WS_U, WS_RHOK, WS_COEF, WS_EBK, WS_RHO, WS_W, WS_MISC, WS_PART,
   WS_OMEGA, WS_DOS, WS_LKEYS, WS_HF, WS_HF2, WS_MU, WS_BANDS2,
-  WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_VU, WS_VB, WS_VX, WS_VT, WS_VG, WS_ONES, WS_SCFY, WS_AND, WS_EXCH, WS_HFPART, WS_BDG, WS_BDGE, WS_BDGI, WS_BDGK, WS_BDGP, WS_BDGB, WS_CSC, WS_UNIW, WS_SPAN, WS_GRAD, WS_GRADE, WS_HFPART2, WS_GEMMSPLIT, WS_GRAM, WS_TSP, WS_TSB, WS_TSV2
+  WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_VU, WS_VB, WS_VX, WS_VT, WS_VG, WS_ONES, WS_SCFY, WS_AND, WS_EXCH, WS_HFPART, WS_BDG, WS_BDGE, WS_BDGI, WS_BDGK, WS_BDGP, WS_BDGB, WS_CSC, WS_UNIW, WS_SPAN, WS_GRAD, WS_GRADE, WS_HFPART2, WS_GEMMSPLIT, WS_GRAM, WS_TSP, WS_TSB, WS_TSV2,
+  WS_STV, WS_STZ, WS_STU, WS_STI
 };
-static_assert(WS_TSV2 < 52, "workspace slots");
+static_assert(WS_STI < 64, "workspace slots");
 
 }  // namespace
 #include "lqm_comm.inc"
@@ -313,8 +316,11 @@ int eigh_threads(int n) { return n <= 16 ? 32 : (n <= 32 ? 64 : (n < 64 ? 128 : 
 // The block size of the one-CTA eigensolver for order n on this context: the value
 // set by lqm_ctx_set_eigh_threads / lqm_autotune_eigh, else the rule above.
 int eigh_threads_for(const lqm_ctx* ctx, int n) {
-  const auto it = ctx->eigh_nt.find(n);
-  return it != ctx->eigh_nt.end() ? it->second : eigh_threads(n);
+  for (const auto* m : {&ctx->eigh_nt, &ctx->eigh_nt_alt}) {
+    const auto it = m->find(n);
+    if (it != m->end()) return it->second;
+  }
+  return eigh_threads(n);
 }
 
 // eigh_kernel instantiation for a block size.  Blocks of up to 128 threads
@@ -775,16 +781,134 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   ctx->eigh_launches++;
 }
 
-// Eigen pass over nk device k-points: bands (n x nk), optionally U and/or rho_k.
-void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
-                 const RhoOut* ro = nullptr) {
-  NvtxRange nvtx_("eigen pass");
-  const int n = (int)H->n;
-  if (use_blocked(ctx, n, (int)H->nR)) {
-    launch_eigh_large(ctx, H, nk, d_ks, d_bands, d_U, ro ? ro->rhok : nullptr, ro ? ro->ebk : nullptr,
-                      ro ? ro->w : nullptr, ro ? ro->mu : 0.0, ro ? ro->T : 0.0);
-    return;
+// ---- staged path (lqm_staged.cuh) ----
+template <class F>
+void set_smem(F* fn, size_t bytes) {
+  ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attr");
+}
+
+template <int WR, int WC, int NB, int KEPT, int MINB>
+void launch_st_hetrd(lqm_ctx* ctx, const StHetrdArgs& a) {
+  const size_t sm = st_hetrd_complex<StGrid<WR, WC, NB, KEPT>>(a.nR) * sizeof(double2);
+  set_smem(st_hetrd_kernel<WR, WC, NB, KEPT, MINB>, sm);
+  st_hetrd_kernel<WR, WC, NB, KEPT, MINB><<<(unsigned)a.nk, 32 * WR * WC, sm, ctx->stream>>>(a);
+}
+
+template <int NB, int MINB>
+void launch_st_hetrd_warp(lqm_ctx* ctx, const StHetrdArgs& a) {
+  constexpr int WPC = 4;
+  const size_t sm = WPC * st_hetrd_complex<StGrid<1, 1, NB, 0>>(a.nR) * sizeof(double2);
+  set_smem(st_hetrd_warp_kernel<NB, WPC, MINB>, sm);
+  st_hetrd_warp_kernel<NB, WPC, MINB><<<(unsigned)((a.nk + WPC - 1) / WPC), 32 * WPC, sm, ctx->stream>>>(a);
+}
+
+template <int NT, int RT, int RR, int MINB>
+void launch_st_dc(lqm_ctx* ctx, const StDcArgs& a) {
+  const size_t sm = st_dc_doubles(a.n, a.Z != nullptr) * sizeof(double);
+  set_smem(st_dc_kernel<NT, RT, RR, MINB>, sm);
+  st_dc_kernel<NT, RT, RR, MINB><<<(unsigned)a.nk, NT, sm, ctx->stream>>>(a);
+}
+
+template <int RT, int MINB>
+void launch_st_back(lqm_ctx* ctx, const StBackArgs& a) {
+  set_smem(st_back_kernel<RT, MINB>, st_back_smem(RT));
+  st_back_kernel<RT, MINB><<<(unsigned)(a.nk * a.groups), 32 * kStBackWarps, st_back_smem(RT), ctx->stream>>>(a);
+}
+
+void launch_eigh_one(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
+                     const RhoOut* ro, const int* only = nullptr);
+
+// Batches of about 4 GB of work buffers.
+void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands,
+                        double2* d_U, const RhoOut* ro) {
+  NvtxRange nvtx_("eigen pass (staged)");
+  const int n = (int)H->n, nR = (int)H->nR;
+  const int64_t nn = (int64_t)n * n;
+  const bool vec = d_U || ro;
+  const int P = st_panels(n);
+  const double per_k = 16.0 * nn + 32.0 * n + (vec ? 24.0 * nn + 1024.0 * P + 8.0 * n : 0.0);
+  const int64_t B = std::min<int64_t>(nk, std::max<int64_t>(32, (int64_t)(4.0e9 / per_k)));
+  double2* V = (double2*)ws_get(ctx, WS_STV, (size_t)B * (nn + 2 * n) * sizeof(double2));
+  double2* tau = V + B * nn;
+  double* d = (double*)(tau + B * n);
+  double* e = d + B * n;
+  // integers: redo flags and their count | ncol | comp
+  int* redo = (int*)ws_get(ctx, WS_STI, (size_t)(3 * B + 1) * sizeof(int));
+  int* ncol = redo + B + 1;
+  int* comp = ncol + B;
+  double *Z = nullptr, *occ = nullptr;
+  double2 *Tm = nullptr, *Uw = nullptr;
+  if (vec) {
+    Tm = (double2*)ws_get(ctx, WS_STZ, (size_t)B * (P * kStNB * kStNB * sizeof(double2) + (nn + n) * sizeof(double)));
+    Z = (double*)(Tm + B * P * kStNB * kStNB);
+    occ = Z + B * nn;
+    if (!d_U) Uw = (double2*)ws_get(ctx, WS_STU, (size_t)B * nn * sizeof(double2));
   }
+  unsigned long long* phases = ctx->phases_on ? ctx->d_phase : nullptr;
+  std::pair<cudaEvent_t, cudaEvent_t> evs{};
+  if (ctx->stats_on) { evs = stat_events(ctx); ck(cudaEventRecord(evs.first, ctx->stream), "event"); }
+  for (int64_t k0 = 0; k0 < nk; k0 += B) {
+    const int64_t nb = std::min(B, nk - k0);
+    double* bands = d_bands + k0 * n;
+    double2* U = d_U ? d_U + k0 * nn : Uw;
+    ck(cudaMemsetAsync(redo, 0, (size_t)(nb + 1) * sizeof(int), ctx->stream), "memset");
+    const StHetrdArgs ha{n, nR, H->d, H->blocks, H->keys, nb, d_ks + k0 * H->d, V, tau, d, e, phases};
+    if (n <= 8) launch_st_hetrd_warp<1, 6>(ctx, ha);
+    else if (n <= 16) launch_st_hetrd_warp<2, 6>(ctx, ha);
+    else if (n <= 24) launch_st_hetrd_warp<3, 4>(ctx, ha);
+    else if (n <= 32) launch_st_hetrd_warp<4, 3>(ctx, ha);
+    else if (n <= 48) launch_st_hetrd<2, 2, 3, 0, 4>(ctx, ha);
+    else if (n <= 64) launch_st_hetrd<2, 2, 4, 0, 3>(ctx, ha);
+    else if (n <= 80) launch_st_hetrd<2, 2, 5, 10, 3>(ctx, ha);
+    else if (n <= 96) launch_st_hetrd<2, 2, 6, 22, 3>(ctx, ha);
+    else if (n <= 112) launch_st_hetrd<2, 2, 7, 14, 2>(ctx, ha);
+    else if (n <= 128) launch_st_hetrd<2, 2, 8, 30, 2>(ctx, ha);
+    else launch_st_hetrd<2, 2, 9, 46, 2>(ctx, ha);
+    RhoOut rk{};
+    if (ro) rk = RhoOut{ro->rhok + k0 * nn, ro->ebk + k0, ro->w + k0, ro->mu, ro->T};
+    const bool part = ro && !d_U;  // only the columns that carry rho_k
+    const StDcArgs da{n, st_depth(n), nb, d, e, bands, Z, rk.mu, rk.T, rk.w, part ? rk.ebk : nullptr, occ, ncol, comp,
+                      redo, phases};
+    if (n <= 32) launch_st_dc<32, 1, 4, 16>(ctx, da);
+    else if (n <= 64) launch_st_dc<128, 4, 8, 4>(ctx, da);
+    else if (n <= 96) launch_st_dc<256, 6, 12, 2>(ctx, da);
+    else launch_st_dc<512, 10, 18, 1>(ctx, da);
+    ctx->launches += 2;
+    ck(cudaGetLastError(), "staged reduction launch");
+    if (vec) {
+      const int cols = 8 * kStBackWarps;
+      const StBackArgs ba{n, nb, V, tau, Tm, Z, ncol, U, (n + cols - 1) / cols, phases};
+      st_tfac_kernel<<<(unsigned)((nb * P + 3) / 4), 128, 0, ctx->stream>>>(ba);
+      if (n <= 32) launch_st_back<4, 3>(ctx, ba);
+      else if (n <= 64) launch_st_back<8, 2>(ctx, ba);
+      else if (n <= 96) launch_st_back<12, 2>(ctx, ba);
+      else if (n <= 128) launch_st_back<16, 1>(ctx, ba);
+      else launch_st_back<18, 1>(ctx, ba);
+      ctx->launches += 3;
+      if (part) {
+        const int64_t nt = (n + 31) / 32;
+        const StRhoArgs oa{n, nb, U, occ, ncol, comp, rk.rhok, phases};
+        st_rho_kernel<<<(unsigned)(nb * (nt * (nt + 1) / 2)), 128, 0, ctx->stream>>>(oa);
+        ctx->launches += 1;
+      } else if (ro) {
+        const int g = (int)std::min<int64_t>(nb, (int64_t)ctx->num_sms * 8);
+        rhok_kernel<<<(unsigned)g, 256, (size_t)(n + 32) * sizeof(double), ctx->stream>>>(
+            n, nb, U, bands, rk.mu, nullptr, rk.T, rk.w, rk.rhok, rk.ebk);
+        ctx->launches += 1;
+      }
+      ck(cudaGetLastError(), "staged back-transformation launch");
+    }
+    // k-points of which a leaf did not converge (none in practice)
+    launch_eigh_one(ctx, H, nb, d_ks + k0 * H->d, bands, d_U ? U : nullptr, ro ? &rk : nullptr, redo);
+  }
+  if (ctx->stats_on) { ck(cudaEventRecord(evs.second, ctx->stream), "event"); ctx->ev_pending.push_back(evs); }
+}
+
+// The one-CTA eigensolver (eigh_kernel) over nk k-points, or over those of them with
+// only[k] != 0 (their count in only[nk]; a few at most, so one CTA per SM).
+void launch_eigh_one(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
+                     const RhoOut* ro, const int* only) {
+  const int n = (int)H->n;
   const DCPlan& plan = get_plan(ctx, n);
   const int nt = eigh_threads_for(ctx, n);
   EighSmemLayout Ls = eigh_smem_layout(n, (int)H->nR, nt, 1);
@@ -798,7 +922,7 @@ void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks
   if (per_sm < 1) fail(LQM_EINVAL, "eigh kernel cannot be resident for n=%d", n);
   const bool need_uwork = ro && !d_U && !a_in_smem;
   const int64_t slot = eigh_slot_doubles(n, a_in_smem, need_uwork);
-  int64_t grid = std::min<int64_t>(nk, (int64_t)per_sm * ctx->num_sms);
+  int64_t grid = std::min<int64_t>(nk, (int64_t)(only ? 1 : per_sm) * ctx->num_sms);
   // keep the scratch below ~16 GB
   const int64_t max_slots = std::max<int64_t>(1, (int64_t)(16.0e9 / (8.0 * (double)slot)));
   grid = std::max<int64_t>(1, std::min(grid, max_slots));
@@ -813,13 +937,45 @@ void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks
   a.mu = ro ? ro->mu : 0.0;
   a.T = ro ? ro->T : 0.0;
   a.phase_cycles = ctx->phases_on ? ctx->d_phase : nullptr;
-  std::pair<cudaEvent_t, cudaEvent_t> evs{};
-  if (ctx->stats_on) { evs = stat_events(ctx); ck(cudaEventRecord(evs.first, ctx->stream), "event"); }
+  a.only = only;
   kfn<<<(unsigned)grid, nt, Ls.total, ctx->stream>>>(a);
   ck(cudaGetLastError(), "eigh_kernel launch");
+  ctx->launches++;
+}
+
+// Eigen pass over nk device k-points: bands (n x nk), optionally U and/or rho_k.
+bool use_staged(const lqm_ctx* ctx, int n, int nR);
+void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
+                 const RhoOut* ro = nullptr) {
+  NvtxRange nvtx_("eigen pass");
+  const int n = (int)H->n;
+  if (use_blocked(ctx, n, (int)H->nR)) {
+    launch_eigh_large(ctx, H, nk, d_ks, d_bands, d_U, ro ? ro->rhok : nullptr, ro ? ro->ebk : nullptr,
+                      ro ? ro->w : nullptr, ro ? ro->mu : 0.0, ro ? ro->T : 0.0);
+    return;
+  }
+  if (use_staged(ctx, n, (int)H->nR)) {
+    launch_eigh_staged(ctx, H, nk, d_ks, d_bands, d_U, ro);
+    ctx->eigh_launches++;
+    return;
+  }
+  std::pair<cudaEvent_t, cudaEvent_t> evs{};
+  if (ctx->stats_on) { evs = stat_events(ctx); ck(cudaEventRecord(evs.first, ctx->stream), "event"); }
+  launch_eigh_one(ctx, H, nk, d_ks, d_bands, d_U, ro);
   if (ctx->stats_on) { ck(cudaEventRecord(evs.second, ctx->stream), "event"); ctx->ev_pending.push_back(evs); }
   ctx->eigh_launches++;
-  ctx->launches++;
+}
+
+// The staged path serves 3 <= n <= kStMaxN unless the context names another path
+// (lqm_ctx_set_eigh_threads, lqm_ctx_set_blocked_min_n).  Measured on B200 against the
+// one-CTA kernel, whole calls (rho / bands, 32, 592 and 4096 k-points): n = 8: 1.25, 1.17,
+// 1.29 / 1.58, 1.56, 1.55 times as fast; n = 33: 1.33, 1.40, 2.15 / 1.72, 1.47, 1.82;
+// n = 64: 1.37, 2.80, 4.17 / 1.15, 2.94, 3.84; n = 96: 1.56, 2.45, 3.15 / 1.37, 2.40, 2.91;
+// n = 144: 1.93, 2.48, 2.72 / 1.45, 2.18, 2.32.  At n = 2 its further launches cost more
+// than they save (0.73 to 1.14 / 0.91 to 1.03).  More than 512 keys: their phases, kept in
+// shared memory per k-point, would take the place of whole CTAs.
+bool use_staged(const lqm_ctx* ctx, int n, int nR) {
+  return n >= 3 && n <= kStMaxN && nR <= 512 && ctx->blocked_min_n == 0 && !ctx->eigh_nt.count(n);
 }
 
 // Path choice: the blocked path from n = 224 on, or from ctx->blocked_min_n when
@@ -1052,15 +1208,26 @@ void check_precision(int precision) {
 // ============================================================================
 namespace {
 
-// One eigen pass over the k-points of several models of uneven order (the one-CTA
-// eigensolver's orders) as ONE launch of eigh_multi_kernel: model m's k-points go to
+// One eigen pass over the k-points of several models of uneven order (below the
+// blocked path).  Orders that the staged path serves run there, model after model;
+// else all of them are ONE launch of eigh_multi_kernel: model m's k-points go to
 // teams of its own block size, several teams per CTA on named barriers.  Writes
 // each model's bands and rho_k batch (with the band energies per k).
 void launch_eigh_multi(lqm_ctx* ctx, int nm, const lqm_hops* const* H, int64_t nk, const double* d_ks,
                        double* const* bands, double2* const* rhok, double* const* ebk, const double* d_w, double mu,
                        double T) {
-  NvtxRange nvtx_("eigen pass (several models, one launch)");
+  NvtxRange nvtx_("eigen pass (several models)");
   if (nm < 1 || nm > kMaxModels) fail(LQM_EINVAL, "between 1 and %d models per launch", kMaxModels);
+  bool staged = true;
+  for (int m = 0; m < nm; ++m) staged = staged && use_staged(ctx, (int)H[m]->n, (int)H[m]->nR);
+  if (staged) {
+    for (int m = 0; m < nm; ++m) {
+      const RhoOut ro{rhok[m], ebk[m], d_w, mu, T};
+      launch_eigh_staged(ctx, H[m], nk, d_ks, bands[m], nullptr, &ro);
+    }
+    ctx->eigh_launches++;  // one pass over all models
+    return;
+  }
   int tnt[kMaxModels];
   int NT = 0;
   for (int m = 0; m < nm; ++m) {
@@ -1254,6 +1421,7 @@ int lqm_ctx_scf_exchange_energy(const lqm_ctx* ctx, double* eJ) {
 
 int lqm_ctx_set_eigh_threads(lqm_ctx* ctx, int64_t n, int nt) {
   if (!ctx || n < 1 || nt < 0 || nt > 512 || nt % 32 != 0) return LQM_EINVAL;
+  ctx->eigh_nt_alt.erase((int)n);
   if (nt == 0) ctx->eigh_nt.erase((int)n);
   else ctx->eigh_nt[(int)n] = nt;
   return LQM_OK;

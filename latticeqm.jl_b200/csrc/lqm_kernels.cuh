@@ -60,6 +60,7 @@ struct EighArgs {
   const double* w;        // nk weights (with rhok)
   double mu, T;
   unsigned long long* phase_cycles;  // [16] per-phase SM cycles summed over CTAs, or null
+  const int* only = nullptr;  // or: solve only the k-points with only[k] != 0, only[nk] of them
 };
 
 enum { PH_BLOCH = 0, PH_HETRD = 1, PH_DC = 2, PH_BACK = 3, PH_OUT = 4, PH_DCSUB = 5, PH_COUNT = 16 };
@@ -213,7 +214,9 @@ __global__ void __launch_bounds__(NT, MINB) eigh_kernel(EighArgs a) {
   double* slot = a.scratch + (int64_t)blockIdx.x * a.slot_doubles;
   EighProf P;
   P.on = a.phase_cycles != nullptr;
-  for (int64_t k = blockIdx.x; k < a.nk; k += gridDim.x) eigh_point(T, a, k, smem, slot, P);
+  if (a.only && a.only[a.nk] == 0) return;
+  for (int64_t k = blockIdx.x; k < a.nk; k += gridDim.x)
+    if (!a.only || a.only[k]) eigh_point(T, a, k, smem, slot, P);
   if (P.on && T.tid == 0) {
     for (int i = 0; i < 5; ++i) atomicAdd(&a.phase_cycles[i], P.acc[i]);
     for (int i = 0; i < 8; ++i) atomicAdd(&a.phase_cycles[PH_DCSUB + i], P.dsub[i]);
