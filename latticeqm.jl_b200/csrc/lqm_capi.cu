@@ -1100,52 +1100,29 @@ void eigh_sharded(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_k
 // Chemical potential entirely on the device: mu_out (device double) receives
 // mu and err_out (device double, cleared here) counts failed searches.  No host
 // synchronisation, so the sequence can be captured in a CUDA graph.
-// WS_MISC layout (64 doubles): [0,1] min/max, [4..13] MuState, [16] mu,
-// [17,18] order statistics, [19] error count, [40..44] SCF scalars.
+// WS_MISC layout (64 doubles): [16] mu, [19] error count, [40..44] SCF scalars.
 void chempot_enqueue(lqm_ctx* ctx, int64_t n, int64_t nk, const double* d_bands, const double* d_w, double filling,
                      double T, double* mu_out, double* err_out) {
   const int64_t nv = n * nk;
-  double* mm = (double*)ws_get(ctx, WS_MISC, 64 * sizeof(double));
-  MuState* st = (MuState*)(mm + 4);
   ck(cudaMemsetAsync(err_out, 0, sizeof(double), ctx->stream), "memset");
-  minmax_kernel<<<1, 1024, 0, ctx->stream>>>(d_bands, nv, mm);
+  // about four values per thread, one CTA per SM at most
+  const int64_t G = std::max<int64_t>(1, std::min<int64_t>((nv + 4 * kMuThreads - 1) / (4 * kMuThreads), ctx->num_sms));
+  double* part = (double*)ws_get(ctx, WS_MU, (size_t)(2 * G * kMuPts) * sizeof(double) + 256);
+  MuArgs a;
+  a.bands = d_bands; a.n = (int)n; a.nv = nv; a.w = d_w; a.filling = filling; a.T = T;
+  a.norm = d_w ? 1.0 / (double)n : 1.0 / (double)nv;
+  a.target = T > 0 ? 0 : 1 + (long long)std::floor(filling * (double)(nv - 1));  // chemicalpotential.jl:9-23
+  a.chunk = (nv + G - 1) / G;
+  a.part = part;
+  a.bar = (unsigned*)(part + 2 * G * kMuPts);
+  a.mu = mu_out;
+  a.err = err_out;
+  ck(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), ctx->stream), "memset");
+  void* args[] = {&a};
+  ck(cudaLaunchCooperativeKernel((const void*)mu_search_kernel, dim3((unsigned)G), dim3(kMuThreads), args, 0,
+                                 ctx->stream),
+     "chemical potential launch");
   ctx->launches += 1;
-  const int64_t nbk = std::max<int64_t>(1, std::min<int64_t>((nv + 4095) / 4096, (int64_t)ctx->num_sms * 4));
-  const int64_t chunk = (nv + nbk - 1) / nbk;
-  if (T > 0) {
-    double* part = (double*)ws_get(ctx, WS_MU, (size_t)nbk * sizeof(double));
-    mu_init_kernel<<<1, 1, 0, ctx->stream>>>(st, mm);
-    const double norm = d_w ? 1.0 / (double)n : 1.0 / (double)nv;
-    for (int it = 0; it < 140; ++it) {
-      filling_partial_kernel<<<(unsigned)nbk, 256, 0, ctx->stream>>>(d_bands, (int)n, nv, d_w, st, T, chunk, part);
-      mu_update_kernel<<<1, 32, 0, ctx->stream>>>(part, (int)nbk, st, filling, norm);
-    }
-    mu_store_kernel<<<1, 32, 0, ctx->stream>>>(st, mu_out, err_out);
-    ctx->launches += 2 + 2 * 140;
-    ck(cudaGetLastError(), "chemical potential launch");
-    return;
-  }
-  // T == 0: midpoint of order statistics i, i+1 (1-based), chemicalpotential.jl:9-23
-  if (filling >= 1.0 || filling <= 0.0) {
-    mu_special_kernel<<<1, 32, 0, ctx->stream>>>(mm, mu_out, filling >= 1.0);
-    ctx->launches += 1;
-    ck(cudaGetLastError(), "chemical potential launch");
-    return;
-  }
-  const long long i1 = 1 + (long long)std::floor(filling * (double)(nv - 1));
-  long long* part = (long long*)ws_get(ctx, WS_MU, (size_t)nbk * sizeof(long long));
-  for (int s = 0; s < 2; ++s) {
-    os_init_kernel<<<1, 1, 0, ctx->stream>>>(st, mm, i1 + s);
-    for (int it = 0; it < 140; ++it) {
-      count_partial_kernel<<<(unsigned)nbk, 256, 0, ctx->stream>>>(d_bands, nv, st, chunk, part);
-      os_update_kernel<<<1, 32, 0, ctx->stream>>>(part, (int)nbk, st);
-    }
-    mu_store_kernel<<<1, 32, 0, ctx->stream>>>(st, mm + 17 + s, err_out);
-    ctx->launches += 2 + 2 * 140;
-  }
-  mu_avg_kernel<<<1, 32, 0, ctx->stream>>>(mm + 17, mm + 18, mu_out);
-  ctx->launches += 1;
-  ck(cudaGetLastError(), "order statistic launch");
 }
 
 double chempot_dev(lqm_ctx* ctx, int64_t n, int64_t nk, const double* d_bands, const double* d_w, double filling,
