@@ -187,6 +187,11 @@ void collect_stats(lqm_ctx* ctx) {
   ctx->q2_pending.clear();
 }
 
+// A host thread that sleeps wakes up about 70 us later, which is most of a small call;
+// so the wait polls without sleeping for its first milliseconds (bands of the n = 2 cell on
+// 128 k-points: 60 us a call against 108).
+constexpr double kSpinSeconds = 4e-3;
+
 void wait_stream(lqm_ctx* ctx) {
   const auto t0 = std::chrono::steady_clock::now();
   for (;;) {
@@ -195,7 +200,7 @@ void wait_stream(lqm_ctx* ctx) {
     if (e != cudaErrorNotReady) ck(e, "device execution");
     const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (el > ctx->timeout_s) fail(LQM_ETIMEOUT, "device work exceeded the %.1f s timeout", ctx->timeout_s);
-    std::this_thread::sleep_for(std::chrono::microseconds(20));
+    if (el > kSpinSeconds) std::this_thread::sleep_for(std::chrono::microseconds(20));
   }
   ck(cudaGetLastError(), "kernel launch");
   collect_stats(ctx);
@@ -1162,9 +1167,10 @@ T* upload(lqm_ctx* ctx, int slot, const T* h, size_t count) {
 }
 
 double* uniform_weights(lqm_ctx* ctx, int64_t nk, int slot = WS_W) {
-  std::vector<double> w((size_t)nk, 1.0 / (double)nk);
-  double* d = upload(ctx, slot, w.data(), w.size());
-  wait_stream(ctx);
+  double* d = (double*)ws_get(ctx, slot, (size_t)nk * sizeof(double));
+  fill_kernel<<<(unsigned)std::min<int64_t>((nk + 255) / 256, 1024), 256, 0, ctx->stream>>>(d, nk, 1.0 / (double)nk);
+  ck(cudaGetLastError(), "fill launch");
+  ctx->launches += 1;
   return d;
 }
 

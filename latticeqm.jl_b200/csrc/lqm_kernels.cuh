@@ -348,6 +348,10 @@ __global__ void __launch_bounds__(128) csc_scatter_kernel(int64_t n, const int64
   }
 }
 
+__global__ void __launch_bounds__(256) fill_kernel(double* x, int64_t m, double v) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) x[i] = v;
+}
+
 // Fixed-order sum of x[0..m) into out[0] (single CTA).
 __global__ void ordered_sum_kernel(const double* __restrict__ x, int64_t m, double* out, int accumulate) {
   __shared__ double red[32];
