@@ -275,9 +275,9 @@ enum WsSlot {
   WS_SCRATCH = 0, WS_KS, WS_BANDS, WS_U, WS_RHOK, WS_COEF, WS_EBK, WS_RHO, WS_W, WS_MISC, WS_PART,
   WS_OMEGA, WS_DOS, WS_LKEYS, WS_HF, WS_HF2, WS_MU, WS_BANDS2,
   WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_VU, WS_VB, WS_VX, WS_VT, WS_VG, WS_ONES, WS_SCFY, WS_AND, WS_EXCH, WS_HFPART, WS_BDG, WS_BDGE, WS_BDGI, WS_BDGK, WS_BDGP, WS_BDGB, WS_CSC, WS_UNIW, WS_SPAN, WS_GRAD, WS_GRADE, WS_HFPART2, WS_GEMMSPLIT, WS_GRAM, WS_TSP, WS_TSB, WS_TSV2,
-  WS_STV, WS_STZ, WS_STU, WS_STI
+  WS_STV, WS_STZ, WS_STU, WS_STI, WS_STOCC
 };
-static_assert(WS_STI < 64, "workspace slots");
+static_assert(WS_STOCC < 64, "workspace slots");
 
 }  // namespace
 #include "lqm_comm.inc"
@@ -835,6 +835,22 @@ void launch_st_back(lqm_ctx* ctx, const StBackArgs& a) {
 void launch_eigh_one(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
                      const RhoOut* ro, const int* only = nullptr);
 
+// rho_k = U f(eps - mu) U^H of nk k-points from all their eigenvectors (mu from mu_ptr
+// unless null), and the band energies.
+void launch_st_rho_from_U(lqm_ctx* ctx, int n, int64_t nk, const double2* U, const double* bands, double mu,
+                          const double* mu_ptr, double T, const double* w, double2* rhok, double* ebk) {
+  double* occ = (double*)ws_get(ctx, WS_STOCC, (size_t)nk * (n * sizeof(double) + 3 * sizeof(int)));
+  int* first = (int*)(occ + nk * n);
+  int* ncol = first + nk;
+  int* comp = ncol + nk;
+  st_occ_kernel<<<(unsigned)((nk + 3) / 4), 128, 0, ctx->stream>>>(n, nk, bands, mu, mu_ptr, T, w, ebk, occ, first, ncol,
+                                                                  comp);
+  const int64_t nt = (n + 31) / 32;
+  const StRhoArgs a{n, nk, U, first, occ, ncol, comp, rhok, nullptr};
+  st_rho_kernel<<<(unsigned)(nk * (nt * (nt + 1) / 2)), 128, 0, ctx->stream>>>(a);
+  ctx->launches += 2;
+}
+
 // Batches of about 4 GB of work buffers.
 void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands,
                         double2* d_U, const RhoOut* ro) {
@@ -904,14 +920,11 @@ void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const doubl
       ctx->launches += 3;
       if (part) {
         const int64_t nt = (n + 31) / 32;
-        const StRhoArgs oa{n, nb, U, occ, ncol, comp, rk.rhok, phases};
+        const StRhoArgs oa{n, nb, U, nullptr, occ, ncol, comp, rk.rhok, phases};
         st_rho_kernel<<<(unsigned)(nb * (nt * (nt + 1) / 2)), 128, 0, ctx->stream>>>(oa);
         ctx->launches += 1;
       } else if (ro) {
-        const int g = (int)std::min<int64_t>(nb, (int64_t)ctx->num_sms * 8);
-        rhok_kernel<<<(unsigned)g, 256, (size_t)(n + 32) * sizeof(double), ctx->stream>>>(
-            n, nb, U, bands, rk.mu, nullptr, rk.T, rk.w, rk.rhok, rk.ebk);
-        ctx->launches += 1;
+        launch_st_rho_from_U(ctx, n, nb, U, bands, rk.mu, nullptr, rk.T, rk.w, rk.rhok, rk.ebk);
       }
       ck(cudaGetLastError(), "staged back-transformation launch");
     }

@@ -288,32 +288,6 @@ __global__ void __launch_bounds__(256) bloch_kernel(int n, int nR, int dim, cons
   }
 }
 
-// rho_k = U diag(f) U^H per k from eigenvectors in HBM; eband_k = w_k sum_j f_j eps_j.
-__global__ void __launch_bounds__(256) rhok_kernel(int n, int64_t nk, const double2* __restrict__ U,
-                                                   const double* __restrict__ bands, double mu_val,
-                                                   const double* mu_ptr, double T,
-                                                   const double* __restrict__ w, double2* __restrict__ rhok,
-                                                   double* __restrict__ eband_k) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const double mu = mu_ptr ? *mu_ptr : mu_val;  // device-resident mu (SCF) or a host value
-  double* f = (double*)smem;
-  double* red = f + n;
-  const Team Tm = make_team();
-  const int64_t nn = (int64_t)n * n;
-  for (int64_t k = blockIdx.x; k < nk; k += gridDim.x) {
-    double eb = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      const double e = bands[k * n + j];
-      const double fj = fermi(e - mu, T);
-      f[j] = fj;
-      eb += e * fj;
-    }
-    eb = team_sum(Tm, eb, red);
-    if (threadIdx.x == 0) eband_k[k] = w[k] * eb;
-    rho_from_U(Tm, n, U + k * nn, n, f, rhok + k * nn, n);
-  }
-}
-
 // coef[kb*nL + l] = w_k exp(-i 2 pi k.L_l)
 __global__ void fold_coef_kernel(int64_t nb, int dim, const double* __restrict__ ks, const double* __restrict__ w,
                                  int nL, const int64_t* __restrict__ Lkeys, double2* __restrict__ coef) {

@@ -1270,13 +1270,56 @@ __global__ void __launch_bounds__(32 * kStBackWarps, MINB) st_back_kernel(StBack
 struct StRhoArgs {
   int n;
   int64_t nk;
-  const double2* U;   // nk x (n x n), packed columns
+  const double2* U;   // nk x (n x n), the packed columns from column first[k] on (null: 0)
+  const int* first;
   const double* occ;  // nk x n
   const int* ncol;
   const int* comp;
   double2* rho;       // nk x (n x n)
   unsigned long long* phase_cycles;
 };
+
+// Occupations of all n columns of U for st_rho_kernel, a warp per k-point: the same choice
+// of the columns that rho_k needs as the density passes make, and its band energy.
+__global__ void __launch_bounds__(128) st_occ_kernel(int n, int64_t nk, const double* bands, double mu_val,
+                                                     const double* mu_ptr, double T, const double* w, double* eband_k,
+                                                     double* occ, int* first, int* ncol, int* comp) {
+  const int lane = threadIdx.x & 31;
+  const int64_t k = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (k >= nk) return;
+  const double mu = mu_ptr ? *mu_ptr : mu_val;
+  const double* bk = bands + k * n;
+  double eb = 0.0;
+  int full = 0, empty = 0, c0 = n, c1 = -1;
+  for (int c = lane; c < n; c += 32) {
+    const double e = bk[c], f = fermi(e - mu, T);
+    eb += e * f;
+    full += f == 1.0;
+    empty += f == 0.0;
+    if (f != 1.0) c0 = min(c0, c);
+    if (f != 0.0) c1 = max(c1, c);
+  }
+  eb = warp_sum(eb);
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    full += __shfl_xor_sync(0xffffffffu, full, s);
+    empty += __shfl_xor_sync(0xffffffffu, empty, s);
+    c0 = min(c0, __shfl_xor_sync(0xffffffffu, c0, s));
+    c1 = max(c1, __shfl_xor_sync(0xffffffffu, c1, s));
+  }
+  const bool cm = full > empty;
+  const int cbeg = cm ? c0 : 0, cend = cm ? n : c1 + 1;
+  for (int c = cbeg + lane; c < cend; c += 32) {
+    const double f = fermi(bk[c] - mu, T);
+    occ[k * n + (c - cbeg)] = cm ? f - 1.0 : f;
+  }
+  if (lane == 0) {
+    eband_k[k] = w[k] * eb;
+    first[k] = cbeg;
+    ncol[k] = cend - cbeg;
+    comp[k] = cm ? 1 : 0;
+  }
+}
 
 // grid: the lower 32 x 32 blocks of each rho_k, one k-point after the other; four warps of
 // one 16 x 16 quadrant each.
@@ -1296,7 +1339,7 @@ __global__ void __launch_bounds__(128) st_rho_kernel(StRhoArgs a) {
   while (J > I) { J -= I + 1; ++I; }
   const int K = a.ncol[k];
   const long long t0 = a.phase_cycles ? clock64() : 0;
-  const double2* U = a.U + k * nn;
+  const double2* U = a.U + k * nn + (a.first ? a.first[k] * n : 0);
   const double* w = a.occ + k * n;
   auto issue = [&](int c0, int b) {
     for (int u = threadIdx.x; u < 32 * KS; u += 128) {
