@@ -615,7 +615,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
       ts_band_kernel<<<nbk, kBlkThreads, 0, ctx->stream>>>(n, A, Bd);
       ck(cudaFuncSetAttribute(ts_chase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsChaseSmem),
          "smem attr");
-      ts_chase_kernel<<<nbk, kTsChaseWarps * 32, kTsChaseSmem, ctx->stream>>>(
+      ts_chase_kernel<<<nbk, kTsPairs * 64, kTsChaseSmem, ctx->stream>>>(
           n, Bd, V2, tau2, dd, ee, ctx->d_err, ctx->dev_wait_limit > 0 ? ctx->dev_wait_limit : kTsWaitPolls);
       ctx->err_armed = true;
       ctx->launches += 2;

@@ -720,7 +720,6 @@ __global__ void __launch_bounds__(kBlkThreads) blk_add_identity_kernel(int n, do
 // ---- Two-stage reduction (lqm_twostage.cuh) ----
 constexpr int kTsB = 16;              // half-bandwidth of the stage-1 band
 constexpr int kTsPanelThreads = 512;  // panel QR: latency-bound row passes, CTA per k-point
-constexpr int kTsChaseWarps = 8;      // bulge chase: sweeps in flight per k-point (one warp each)
 constexpr int kTsWaitPolls = 1 << 26; // bound of one inter-warp wait of the chase (shared-memory polls, ~1 s)
 
 // complex per k-point of the stage-2 reflector store (sweeps 0..n-2, tmax slots of kTsB each)
@@ -746,69 +745,226 @@ __global__ void __launch_bounds__(kBlkThreads) ts_band_kernel(int n, const doubl
   ts_band_extract<kTsB>(T, n, A + b * (int64_t)n * n, n, Bd + b * 2 * kTsB * (int64_t)n);
 }
 
-// grid (B), kTsChaseWarps warps: the bulge chase of one k-point.  Warp w takes the
-// sweeps s = w, w + W, ... (ts_chase_sweep, its blocks in the warp's window of
-// dynamic shared memory); before task t of sweep s it waits until sweep s - 1 has
-// finished its tasks 0 .. t + 2 (the tasks whose rows and columns overlap task t's),
-// read from a per-warp progress word in shared memory.  The band stays in global
-// memory (L1/L2): a warp's stores are fenced at block scope before it publishes
-// progress, and a waiting warp fences after it reads it.  Every wait is bounded
-// (wait_polls polls of the progress word): on expiry the kernel records an error in
-// *err, every warp stops at its next wait, and d / e are written as zeros.  V2 / tau2 (or null): the reflectors for the
-// back-transformation.  Outputs: d (n) and e (n - 1) of the real tridiagonal.
-constexpr int kTsWin = 3 * kTsB * (kTsB + 1) + 2 * kTsB;  // complex per warp window
-constexpr int kTsChaseSmem = kTsChaseWarps * kTsWin * 16;
-__global__ void __launch_bounds__(kTsChaseWarps * 32) ts_chase_kernel(int n, double2* Bd, double2* V2,
-                                                                      double2* tau2, double* d, double* e,
-                                                                      int* err, long long wait_polls) {
+// Bulge chase of one k-point (the tasks of ts_chase_sweep): grid (B), kTsPairs pairs of
+// warps; pair p takes the sweeps s = p, p + kTsPairs, ...  Before task t of sweep s the pair
+// waits until sweep s - 1 has finished its tasks 0 .. t + 2 (those whose rows and columns
+// overlap task t's), read from a per-pair progress word in shared memory.
+// A pair is a two-stage pipeline over the tasks of its sweep.  The maker takes task t's
+// column x, forms the reflector v and applies it to the block E below (E <- E H), which
+// holds the next task's x, and so runs along the only chain within a sweep; the applier,
+// one task behind at most, applies v to the rest F of the block that the task started
+// from and two-sided to the diagonal block D, writes both back and publishes the task.
+// They meet on the pair's named barrier once per task.  E passes through three buffers in
+// shared memory (row by lane pair in the maker, column by lane pair in the applier); D and
+// E live in registers while they are changed; rows past the matrix's end are zeros.
+// The band stays in global memory (L1/L2): the applier's stores are fenced at block scope
+// before it publishes, and a waiting warp fences after it reads the progress word.  Every
+// wait is bounded (wait_polls polls): on expiry the kernel records an error in *err, every
+// pair stops at its next task, and d / e are written as zeros.  V2 / tau2 (or null): the
+// reflectors for the back-transformation.  Outputs: d (n) and e (n - 1) of the real
+// tridiagonal.  Bound by the latency of a task: 3 n of them follow each other at least.  One warp
+// per sweep that did a whole task by itself (1560 instructions) took 44 ms at n = 1324 for up
+// to 148 k-points; with pairs whole calls went from 12.2 to 9.0 ms (bands, n = 364, 32 k-points) and from 155 to 135 ms
+// (n = 1324, 100).  Eight pairs of 128 registers a thread; ten of 96 spill.
+constexpr int kTsPairs = 8;
+constexpr int kTsLw = kTsB + 1;  // block pitch (odd: row and column walks conflict-free)
+constexpr int kTsBlk = kTsB * kTsLw;
+constexpr int kTsPairWin = 4 * kTsBlk + 3 * kTsB + 4;  // three E buffers, D | v (2), w | tau, beta (2 each)
+constexpr int kTsChaseSmem = kTsPairs * kTsPairWin * 16;
+static_assert(kTsChaseSmem <= 225 * 1024, "chase windows exceed shared memory");
+static_assert(kTsB == 16, "a lane pair per row or column, eight elements each");
+
+__device__ __forceinline__ double ts_warp_sum(double v) {  // every lane gets the sum (two tensor steps)
+  double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+  dmma_884(a0, a1, 1.0, v);
+  dmma_884(b0, b1, 1.0, a0 + a1);
+  return b0;
+}
+__device__ __forceinline__ double2 ts_pair_add(double2 v) {  // + the value of lane ^ 16
+  v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+  v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+  return v;
+}
+
+__global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, double2* Bd, double2* V2, double2* tau2,
+                                                                    double* d, double* e, int* err,
+                                                                    long long wait_polls) {
   extern __shared__ __align__(16) double2 tswin[];
-  __shared__ long long prog[kTsChaseWarps];
+  __shared__ long long prog[kTsPairs];
   __shared__ int stop;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const WarpTeam T = make_warpteam();
+  __shared__ int halt[kTsPairs];  // the maker gave up (read by the applier after their barrier)
+  constexpr int B = kTsB, LW = kTsLw, ldb = 2 * B;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, pair = w >> 1;
+  const bool maker = (w & 1) == 0;
+  const int r = lane & 15, hh = lane >> 4;
   const int64_t b = blockIdx.x;
-  constexpr int ldb = 2 * kTsB;
   double2* Bk = Bd + b * ldb * (int64_t)n;
-  const int tmax = ts_tmax(n, kTsB);
+  double2* buf = tswin + pair * kTsPairWin;  // block i at buf + i kTsBlk, (row, column) at row + LW column
+  double2* Dm = buf + 3 * kTsBlk;            // the part of D above the diagonal, by rows of its mirror
+  double2* vb = Dm + kTsBlk;                 // v of even and odd tasks
+  double2* wv = vb + 2 * B;
+  double2* sc = wv + B;                      // tau, (beta, 0) of even and odd tasks
+  const int tmax = ts_tmax(n, B);
   const long long unit = tmax + 1;  // progress: s * unit + tasks done
-  if (lane == 0) prog[w] = -1;
+  if (threadIdx.x < kTsPairs) { prog[threadIdx.x] = -1; halt[threadIdx.x] = 0; }
   if (threadIdx.x == 0) stop = (err && *(volatile int*)err) ? 1 : 0;
   __syncthreads();
   volatile long long* vprog = prog;
   volatile int* vstop = &stop;
-  bool ok = *vstop == 0;
-  const int wp = (w + kTsChaseWarps - 1) % kTsChaseWarps;  // the warp of sweep s - 1
-  for (int s = w; ok && s <= n - 2; s += kTsChaseWarps) {
-    const int ntp = (s > 0) ? ts_tasks(n, kTsB, s - 1) : 0;
-    auto wait = [&](int t) -> bool {
-      if (s == 0) return true;
-      const long long need = (long long)(s - 1) * unit + (t + 3 < ntp ? t + 3 : ntp);
-      bool good = true;
-      if (lane == 0) {
-        long long polls = 0;
-        while (vprog[wp] < need) {
-          if (*vstop) { good = false; break; }
-          if (++polls > wait_polls) {
-            *vstop = 1;
-            if (err) atomicExch(err, 2);
-            good = false;
-            break;
-          }
-        }
-      }
-      good = __shfl_sync(0xffffffffu, good, 0);
-      __syncwarp();
-      __threadfence_block();
-      return good;
-    };
-    auto done = [&](int t) {
-      __threadfence_block();
-      __syncwarp();
-      if (lane == 0) vprog[w] = (long long)s * unit + t + 1;
-    };
-    double2* vo = V2 ? V2 + b * ts_v2_stride(n) + (int64_t)s * tmax * kTsB : nullptr;
+  const int pp = (pair + kTsPairs - 1) % kTsPairs;  // the pair of sweep s - 1
+  auto meet = [&] { asm volatile("bar.sync %0, 64;\n" ::"r"(1 + pair) : "memory"); };
+  const bool go = *vstop == 0;
+  int it = 0;  // tasks of this pair so far: the buffers' turn (the maker's next sweep overlaps the applier's last task)
+  for (int s = pair; go && s <= n - 2; s += kTsPairs) {
+    const int nt = ts_tasks(n, B, s), ntp = s > 0 ? ts_tasks(n, B, s - 1) : 0;
+    double2* vo = V2 ? V2 + b * ts_v2_stride(n) + (int64_t)s * tmax * B : nullptr;
     double2* to = tau2 ? tau2 + b * ts_tau2_stride(n) + (int64_t)s * tmax : nullptr;
-    ok = ts_chase_sweep<kTsB>(T, n, s, Bk, vo, to, tswin + w * kTsWin, wait, done);
+    bool ok = true;
+    if (maker) {
+      for (int t = 0; t < nt; ++t, ++it) {
+        // R0: first row of the task; rows R0 .. R0 + 15 (zeros past n), E below them
+        const int R0 = s + 1 + t * B, R1 = R0 + B;
+        if (s > 0) {
+          const long long need = (long long)(s - 1) * unit + (t + 3 < ntp ? t + 3 : ntp);
+          if (lane == 0) {
+            long long polls = 0;
+            while (vprog[pp] < need) {
+              if (*vstop) { ok = false; break; }
+              if (++polls > wait_polls) {
+                *vstop = 1;
+                if (err) atomicExch(err, 2);
+                ok = false;
+                break;
+              }
+            }
+          }
+          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+          __threadfence_block();
+        }
+        if (!ok) break;
+        double2 E[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int q = 8 * hh + k;
+          E[k] = (R1 + r < n) ? Bk[(B + r - q) + (int64_t)(R0 + q) * ldb] : cmk(0.0, 0.0);
+        }
+        double2* X = buf + (it % 3) * kTsBlk;  // x: its first column
+        double2 x = cmk(0.0, 0.0);
+        if (t == 0) x = (R0 + r < n) ? Bk[(1 + r) + (int64_t)s * ldb] : cmk(0.0, 0.0);
+        else x = X[r];
+        const double nrm = ts_warp_sum((hh == 0 && r > 0) ? x.x * x.x + x.y * x.y : 0.0);
+        const double2 alpha = shfl_c(x, 0);
+        double2 tj, scal;
+        double beta;
+        zlarfg_scalars(alpha, nrm, &tj, &beta, &scal);
+        const double2 vr = r == 0 ? cmk(1.0, 0.0) : cmul(scal, x);
+        double2* v = vb + (it & 1) * B;
+        if (hh == 0) {
+          v[r] = vr;
+          if (vo) vo[(int64_t)t * B + r] = vr;
+        }
+        if (lane == 0) {
+          sc[2 * (it & 1)] = tj;
+          sc[2 * (it & 1) + 1] = cmk(beta, 0.0);
+          if (to) to[t] = tj;
+        }
+        __syncwarp();
+        // E <- E H: z = E v, E -= tau z v^H
+        double2 vq[8], e0 = cmk(0.0, 0.0), e1 = e0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) vq[k] = v[8 * hh + k];
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          e0 = cfma(e0, E[k], vq[k]);
+          e1 = cfma(e1, E[k + 1], vq[k + 1]);
+        }
+        const double2 z = cmul(tj, ts_pair_add(cadd(e0, e1)));
+        double2* EN = buf + ((it + 1) % 3) * kTsBlk;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) EN[r + LW * (8 * hh + k)] = cfms(E[k], z, cconj(vq[k]));
+        meet();  // v, E and the reflector's scalars are the applier's; it is done with task t - 1
+      }
+      if (!ok) {
+        if (lane == 0) halt[pair] = 1;
+        meet();
+        break;
+      }
+    } else {
+      for (int t = 0; t < nt; ++t, ++it) {
+        meet();
+        if (((volatile int*)halt)[pair]) { ok = false; break; }
+        const int R0 = s + 1 + t * B, c = t == 0 ? s : R0 - B;
+        double2 D[8];  // D(r, 8 hh + k), the lower triangle
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int q = 8 * hh + k;
+          D[k] = (q <= r && R0 + r < n) ? Bk[(r - q) + (int64_t)(R0 + q) * ldb] : cmk(0.0, 0.0);
+        }
+        const double2* v = vb + (it & 1) * B;
+        const double2 tj = sc[2 * (it & 1)], beta = sc[2 * (it & 1) + 1];
+        double2* X = buf + (it % 3) * kTsBlk;
+        // F <- H^H F, column r (1 .. 15), rows 8 hh ..; the first column becomes beta e1
+        if (t > 0) {
+          double2 f[8], vf[8], a0 = cmk(0.0, 0.0), a1 = a0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            f[k] = X[8 * hh + k + LW * r];
+            vf[k] = v[8 * hh + k];
+          }
+#pragma unroll
+          for (int k = 0; k < 8; k += 2) {
+            a0 = cfma_conj(a0, vf[k], f[k]);
+            a1 = cfma_conj(a1, vf[k + 1], f[k + 1]);
+          }
+          const double2 fl = cmul(cconj(tj), ts_pair_add(cadd(a0, a1)));
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            X[8 * hh + k + LW * r] = r > 0 ? cfms(f[k], vf[k], fl) : (hh == 0 && k == 0) ? beta : cmk(0.0, 0.0);
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {  // back to the band, by columns: two at a time
+            const int l = 2 * k + hh;
+            if (R0 + r < n) Bk[(B + r - l) + (int64_t)(c + l) * ldb] = X[r + LW * l];
+          }
+        } else if (hh == 0 && R0 + r < n) {
+          Bk[(1 + r) + (int64_t)s * ldb] = r == 0 ? beta : cmk(0.0, 0.0);
+        }
+        // D <- H^H D H: y = D v, gamma = v^H y, w = tau y - 1/2 |tau|^2 gamma v,
+        // D -= w v^H + v w^H
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int q = 8 * hh + k;
+          if (q < r) Dm[q + LW * r] = cconj(D[k]);
+        }
+        __syncwarp();
+        double2 vq[8], a0 = cmk(0.0, 0.0), a1 = a0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) vq[k] = v[8 * hh + k];
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const int q = 8 * hh + k;
+          a0 = cfma(a0, q <= r ? D[k] : Dm[r + LW * q], vq[k]);
+          a1 = cfma(a1, q + 1 <= r ? D[k + 1] : Dm[r + LW * (q + 1)], vq[k + 1]);
+        }
+        const double2 y = ts_pair_add(cadd(a0, a1)), vr = v[r];
+        const double g = ts_warp_sum(hh == 0 ? cmulc(vr, y).x : 0.0);
+        const double h = -0.5 * (tj.x * tj.x + tj.y * tj.y) * g;
+        const double2 wr = cadd(cmul(tj, y), cscale(h, vr));
+        if (hh == 0) wv[r] = wr;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int q = 8 * hh + k;
+          double2 x = cfms(cfms(D[k], wr, cconj(vq[k])), vr, cconj(wv[q]));
+          if (q == r) x.y = 0.0;
+          if (q <= r && R0 + r < n) Bk[(r - q) + (int64_t)(R0 + q) * ldb] = x;
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) vprog[pair] = (long long)s * unit + t + 1;
+      }
+      if (!ok) break;
+    }
   }
   __syncthreads();
   const bool fin = *vstop == 0;  // after a failed wait: zeros, so the solver that follows stays bounded

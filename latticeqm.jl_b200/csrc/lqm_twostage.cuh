@@ -181,7 +181,8 @@ LQM_FN void ts_band_extract(const TeamT& T, int n, const double2* A, int lda, do
 // task's), and F, x and D go back to the band once they are final.  wait(t) is
 // called before task t's loads (false: give up, the sweep returns false) and done(t)
 // after its stores.  vout / tauout (or null): task t's v (B complex, zero-padded)
-// at vout + t B and tau at tauout[t].  The team is one warp on the device.
+// at vout + t B and tau at tauout[t].  The defining form, against which the emulation
+// checks the device's pipeline of the same tasks (ts_chase_kernel).
 template <int B, class TeamT, class WaitF, class DoneF>
 LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* vout, double2* tauout,
                            double2* win, WaitF wait, DoneF done) {
@@ -228,29 +229,8 @@ LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* v
     team_sync(T);
     for (int r = T.tid; r < L; r += T.nt) EF[r] = (r == 0) ? cmk(beta, 0.0) : cmk(0.0, 0.0);
     const double2 ctj = cconj(tj);
-    // F <- H^H F, column l (1 .. B-1).  Device: lanes l and l + 16 take rows 0..7 and
-    // 8..15 of column l, two partial sums each, added across the lane pair.
+    // F <- H^H F, column l (1 .. B-1)
     if (t > 0) {
-#if defined(__CUDACC__)
-      const int l = T.lane & 15, hh = T.lane >> 4;
-      double2* f = EF + l * LW;
-      double2 a0 = cmk(0.0, 0.0), a1 = cmk(0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const int r0 = 8 * hh + k;
-        if (r0 < L) a0 = cfma_conj(a0, v[r0], f[r0]);
-        if (r0 + 1 < L) a1 = cfma_conj(a1, v[r0 + 1], f[r0 + 1]);
-      }
-      const double2 pp = cadd(a0, a1);
-      const double2 fl = cmul(ctj, cadd(shfl_c(pp, l), shfl_c(pp, l + 16)));
-      if (l >= 1) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int r = 8 * hh + k;
-          if (r < L) f[r] = cfms(f[r], v[r], fl);
-        }
-      }
-#else
       for (int l = 1 + T.tid; l < B; l += T.nt) {
         double2* f = EF + l * LW;
         double2 acc = cmk(0.0, 0.0);
@@ -258,7 +238,6 @@ LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* v
         const double2 fl = cmul(ctj, acc);
         for (int r = 0; r < L; ++r) f[r] = csub(f[r], cmul(v[r], fl));
       }
-#endif
     }
     team_sync(T);
     // x and F are final: back to the band (columns c .. c+B-1, rows R0 ..)
@@ -268,54 +247,7 @@ LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* v
       if (r < L) *ts_bptr(Bd, ldb, R0 + r, c + l) = EF[r + l * LW];
     }
     // D <- H^H D H: y = D v, gamma = v^H y, w = tau y - 1/2 |tau|^2 gamma v; then
-    // E <- E H: z_i = sum_q E(i, q) v_q, E(i, q) -= tau z_i conj(v_q).  Device: lanes
-    // r and r + 16 take columns 0..7 and 8..15 of row r, two partial sums each.
-#if defined(__CUDACC__)
-    {
-      const int r = T.lane & 15, hh = T.lane >> 4;
-      double2 a0 = cmk(0.0, 0.0), a1 = cmk(0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const int q0 = 8 * hh + k, q1 = q0 + 1;
-        if (r < L && q0 < L) a0 = cfma(a0, (q0 <= r) ? D[r + q0 * LW] : cconj(D[q0 + r * LW]), v[q0]);
-        if (r < L && q1 < L) a1 = cfma(a1, (q1 <= r) ? D[r + q1 * LW] : cconj(D[q1 + r * LW]), v[q1]);
-      }
-      const double2 pp = cadd(a0, a1);
-      const double2 yr = cadd(shfl_c(pp, r), shfl_c(pp, r + 16));
-      const double g = warp_sum_bcast((hh == 0 && r < L) ? cmulc(v[r], yr).x : 0.0);
-      const double h = -0.5 * (tj.x * tj.x + tj.y * tj.y) * g;
-      if (hh == 0 && r < L) w[r] = cadd(cmul(tj, yr), cscale(h, v[r]));
-      team_sync(T);  // w complete; every lane has read D
-      if (r < L) {
-        const double2 vr = v[r], wr = w[r];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int q = 8 * hh + k;
-          if (q <= r) {
-            double2 a = cfms(cfms(D[r + q * LW], wr, cconj(v[q])), vr, cconj(w[q]));
-            if (q == r) a.y = 0.0;
-            D[r + q * LW] = a;
-          }
-        }
-      }
-      double2 e0 = cmk(0.0, 0.0), e1 = cmk(0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const int q0 = 8 * hh + k, q1 = q0 + 1;
-        if (r < L2 && q0 < L) e0 = cfma(e0, EN[r + q0 * LW], v[q0]);
-        if (r < L2 && q1 < L) e1 = cfma(e1, EN[r + q1 * LW], v[q1]);
-      }
-      const double2 pe = cadd(e0, e1);
-      const double2 z = cmul(tj, cadd(shfl_c(pe, r), shfl_c(pe, r + 16)));
-      if (r < L2) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int q = 8 * hh + k;
-          if (q < L) EN[r + q * LW] = cfms(EN[r + q * LW], z, cconj(v[q]));
-        }
-      }
-    }
-#else
+    // E <- E H: z_i = sum_q E(i, q) v_q, E(i, q) -= tau z_i conj(v_q)
     double2 yr = cmk(0.0, 0.0);
     double g = 0.0;
     for (int r = T.tid; r < L; r += T.nt) {
@@ -323,17 +255,11 @@ LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* v
       for (int q = 0; q < L; ++q) acc = cadd(acc, cmul((q <= r) ? D[r + q * LW] : cconj(D[q + r * LW]), v[q]));
       yr = acc;
       g += cmulc(v[r], acc).x;
-#if !defined(__CUDACC__)
       w[r] = acc;  // one-thread team: y kept in w until gamma is complete
-#endif
     }
     g = warp_sum_bcast(g);
     const double h = -0.5 * (tj.x * tj.x + tj.y * tj.y) * g;
-#if defined(__CUDACC__)
-    for (int r = T.tid; r < L; r += T.nt) w[r] = cadd(cmul(tj, yr), cscale(h, v[r]));
-#else
     for (int r = 0; r < L; ++r) w[r] = cadd(cmul(tj, w[r]), cscale(h, v[r]));
-#endif
     team_sync(T);  // every thread has read D before it is rewritten
     for (int r = T.tid; r < L; r += T.nt) {
       const double2 vr = v[r], wr = w[r];
@@ -350,7 +276,6 @@ LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* v
       const double2 z = cmul(tj, acc);
       for (int q = 0; q < L; ++q) EN[i + q * LW] = csub(EN[i + q * LW], cmul(z, cconj(v[q])));
     }
-#endif
     team_sync(T);
     for (int idx = T.tid; idx < B * B; idx += T.nt) {
       const int r = idx % B, q = idx / B;
