@@ -709,8 +709,9 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
       // a register window of each column per thread
       std::pair<cudaEvent_t, cudaEvent_t> qev{};
       if (ctx->stats_on) { qev = stat_events(ctx); ck(cudaEventRecord(qev.first, ctx->stream), "event"); }
-      ts_q2g_kernel<<<dim3((unsigned)((K + kTsQ2gThreads - 1) / kTsQ2gThreads), (unsigned)nbk), kTsQ2gThreads, 0,
-                      ctx->stream>>>(n, c0, K, V2, tau2, Ucur);
+      ck(cudaFuncSetAttribute(ts_q2g_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsQ2gSmem), "smem attr");
+      ts_q2g_kernel<<<dim3((unsigned)((K + kTsQ2gThreads - 1) / kTsQ2gThreads), (unsigned)nbk), kTsQ2gThreads,
+                      kTsQ2gSmem, ctx->stream>>>(n, c0, K, V2, tau2, Ucur);
       ctx->launches++;
       if (ctx->stats_on) {
         ck(cudaEventRecord(qev.second, ctx->stream), "event");

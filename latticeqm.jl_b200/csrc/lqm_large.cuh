@@ -975,34 +975,36 @@ __global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, doubl
   }
 }
 
-// Q2 Z in the grouped order (ts_q2_apply_grouped_host): grid (ceil(K / 256), B),
+// Q2 Z in the grouped order (ts_q2_apply_grouped_host): grid (ceil(K / kTsQ2gThreads), B),
 // thread = one of the columns c0 .. c0+K-1 of U (n x n per k-point, in place).
 // Each (group of 16 sweeps, task t) step applies 16 reflectors to a window of 31
 // rows of the thread's column, held in registers (all indices compile-time); the
 // window slides by 16 rows per step, so a group streams the column once.  The
 // step's reflectors and taus (16 x 16 + 16 complex; zeros where a sweep has no
-// task t) are copied into shared memory by cp.async one step ahead, and the 16 rows
-// of the next slide are prefetched into L1.  A reflector's dot product runs in two
-// partial sums: with four the prefetch addresses no longer fit the 255 registers
-// (spills), and two with the prefetch measured 5% faster than four without it.
-constexpr int kTsQ2gThreads = 256;
-// rows r0 .. r0 + kTsB - 1 (those below n) of column c: 256 bytes, at most three lines,
-// requested one step before the slide that loads them, so that they arrive while the
-// step's reflectors are applied
-__device__ __forceinline__ void prefetch_rows(const double2* c, int r0, int n) {
-  if (r0 < n) prefetch_l1(c + r0);
-  if (r0 + 8 < n) prefetch_l1(c + r0 + 8);
-  if (r0 + kTsB - 1 < n) prefetch_l1(c + r0 + kTsB - 1);
-}
+// task t) are copied into shared memory by cp.async one step ahead.
+// Bound by the FP64 pipe (64 FMA per row and reflector pair) as long as the window's
+// traffic stays off it: a column per lane makes every direct access 32 separate lines,
+// as many LSU cycles per step as the arithmetic takes, and all warps at once behind the
+// step's barrier.  So the 16 rows that enter and leave move through a 32-column
+// exchange block per warp, 256 contiguous bytes of a column per half-warp, the entering
+// rows by cp.async one step ahead.
+constexpr int kTsQ2gThreads = 128;
+constexpr int kTsQ2gCtas = 2;
 constexpr int kTsQ2gStep = kTsB * kTsB + kTsB;  // complex per staged step
-__global__ void __launch_bounds__(kTsQ2gThreads, 1) ts_q2g_kernel(int n, int c0, int K, const double2* V2,
-                                                                  const double2* tau2, double2* U) {
-  constexpr int B = kTsB, W = 2 * kTsB - 1;
-  __shared__ __align__(16) double2 sv[2][kTsQ2gStep];
+constexpr int kTsQ2gPitch = kTsB + 1;           // complex per column of the exchange block (conflict-free)
+constexpr int kTsQ2gSmem = (3 * kTsQ2gStep + kTsQ2gThreads * kTsQ2gPitch) * 16;
+__global__ void __launch_bounds__(kTsQ2gThreads, kTsQ2gCtas) ts_q2g_kernel(int n, int c0, int K, const double2* V2,
+                                                                           const double2* tau2, double2* U) {
+  constexpr int B = kTsB, W = 2 * kTsB - 1, P = kTsQ2gPitch;
+  static_assert(B == 16, "a half-warp moves one column's rows");
+  extern __shared__ __align__(16) unsigned char q2g_smem[];
+  double2* sv = (double2*)q2g_smem;  // three steps of reflectors
+  const int lane = threadIdx.x & 31;
+  double2* xb = sv + 3 * kTsQ2gStep + (threadIdx.x >> 5) * 32 * P;  // the warp's exchange block, [column][row]
   const int64_t b = blockIdx.y;
-  const int col = blockIdx.x * kTsQ2gThreads + threadIdx.x;
-  const bool act = col < K;
-  double2* Uc = U + b * (int64_t)n * n + (int64_t)(c0 + (act ? col : 0)) * n;
+  const int cw = blockIdx.x * kTsQ2gThreads + (threadIdx.x & ~31);  // the warp's first column
+  const int xc = lane >> 4, xr = lane & 15;                          // this lane's part of a moved column pair
+  double2* Uw = U + b * (int64_t)n * n + (int64_t)(c0 + cw + xc) * n + xr;
   const double2* Vk = V2 + b * ts_v2_stride(n);
   const double2* tk = tau2 + b * ts_tau2_stride(n);
   const int tmax = ts_tmax(n, B);
@@ -1011,7 +1013,7 @@ __global__ void __launch_bounds__(kTsQ2gThreads, 1) ts_q2g_kernel(int n, int c0,
   const int g0 = (ns - 1) / B;  // highest group
   // step (g, t) -> shared buffer: reflector i of the step = sweep g B + i, task t
   auto stage = [&](int g, int t, double2* dst) {
-    for (int e = threadIdx.x; e < kTsQ2gStep; e += blockDim.x) {
+    for (int e = threadIdx.x; e < kTsQ2gStep; e += kTsQ2gThreads) {
       const int i = (e < B * B) ? e / B : e - B * B;
       const int s = g * B + i;
       const bool ok = s < ns && t < ts_tasks(n, B, s);
@@ -1019,24 +1021,57 @@ __global__ void __launch_bounds__(kTsQ2gThreads, 1) ts_q2g_kernel(int n, int c0,
       cp_async16(dst + e, ok ? (const void*)src : (const void*)Vk, ok);
     }
   };
+  // rows r0 .. r0 + 15 of the warp's columns into / out of the exchange block (rows past
+  // n and columns past K: zeros in, nothing out)
+  auto rows_in = [&](int r0) {
+#pragma unroll 4
+    for (int q = 0; q < 16; ++q) {
+      const bool ok = r0 + xr < n && cw + 2 * q + xc < K;
+      cp_async16(xb + (2 * q + xc) * P + xr, ok ? (const void*)(Uw + r0 + (int64_t)(2 * q) * n) : (const void*)Vk, ok);
+    }
+  };
+  auto rows_out = [&](int r0) {
+#pragma unroll 4
+    for (int q = 0; q < 16; ++q)
+      if (r0 + xr < n && cw + 2 * q + xc < K) Uw[r0 + (int64_t)(2 * q) * n] = xb[(2 * q + xc) * P + xr];
+  };
+  double2* xl = xb + lane * P;  // this lane's column
   int buf = 0;
-  stage(g0, 0, sv[0]);
+  stage(g0, 0, sv);
   cp_async_commit();
   for (int g = g0; g >= 0; --g) {
     const int s0 = g * B;
     const int nt = ts_tasks(n, B, s0);
     double2 z[W];
     const int w0 = s0 + 1;
+    // the group's first window, in two passes of the exchange block
+    rows_in(w0);
+    cp_async_commit();
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
 #pragma unroll
-    for (int j = 0; j < W; ++j) z[j] = (act && w0 + j < n) ? Uc[w0 + j] : cmk(0.0, 0.0);
+    for (int j = 0; j < B; ++j) z[j] = xl[j];
+    __syncwarp();
+    rows_in(w0 + B);
+    cp_async_commit();
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int j = B; j < W; ++j) z[j] = xl[j - B];
+    __syncwarp();
+    if (nt > 1) rows_in(w0 + W);  // the first slide's rows
+    cp_async_commit();
     for (int t = 0; t < nt; ++t) {
-      // next step: (g, t + 1), or the next group's first
-      if (t + 1 < nt) stage(g, t + 1, sv[buf ^ 1]);
-      else if (g > 0) stage(g - 1, 0, sv[buf ^ 1]);
+      // next step: (g, t + 1), or the next group's first.  In flight after this commit, in
+      // order: this step's reflectors, the entering rows, the next step's reflectors.  The
+      // buffer being filled was last read two steps ago, before the last barrier.
+      const int nb = (buf == 2) ? 0 : buf + 1;
+      if (t + 1 < nt) stage(g, t + 1, sv + nb * kTsQ2gStep);
+      else if (g > 0) stage(g - 1, 0, sv + nb * kTsQ2gStep);
       cp_async_commit();
-      cp_async_wait_keep1();
+      asm volatile("cp.async.wait_group 2;\n" ::: "memory");
       __syncthreads();
-      const double2* vs = sv[buf];
+      const double2* vs = sv + buf * kTsQ2gStep;
 #pragma unroll
       for (int i = B - 1; i >= 0; --i) {
         const double2 tj = vs[B * B + i];
@@ -1047,22 +1082,35 @@ __global__ void __launch_bounds__(kTsQ2gThreads, 1) ts_q2g_kernel(int n, int c0,
 #pragma unroll
         for (int r = 0; r < B; ++r) z[i + r] = cfms(z[i + r], vs[i * B + r], f);
       }
-      __syncthreads();  // the buffer is refilled two steps on
-      buf ^= 1;
+      buf = nb;
       const int wt = w0 + t * B;  // first row of this step's window
       if (t + 1 < nt) {
+        cp_async_wait_keep1();  // the entering rows
+        __syncwarp();
+        const double2 zl = z[B - 1];  // leaves too, but its place is taken by the first entering row
 #pragma unroll
-        for (int j = 0; j < B; ++j)
-          if (act && wt + j < n) Uc[wt + j] = z[j];
-#pragma unroll
-        for (int j = 0; j < W - B; ++j) z[j] = z[j + B];
-#pragma unroll
-        for (int j = W - B; j < W; ++j) z[j] = (act && wt + B + j < n) ? Uc[wt + B + j] : cmk(0.0, 0.0);
-        if (act && t + 2 < nt) prefetch_rows(Uc, wt + B + W, n);  // the next step's slide
+        for (int j = 0; j < B; ++j) {  // each lane swaps its own column: row wt + j out, row wt + W + j in
+          const double2 in = xl[j];
+          xl[j] = (j < B - 1) ? z[j] : zl;
+          if (j < W - B) z[j] = z[j + B];
+          z[W - B + j] = in;
+        }
+        __syncwarp();
+        rows_out(wt);
+        __syncwarp();
+        if (t + 2 < nt) rows_in(wt + B + W);
+        cp_async_commit();
       } else {
 #pragma unroll
-        for (int j = 0; j < W; ++j)
-          if (act && wt + j < n) Uc[wt + j] = z[j];
+        for (int j = 0; j < B; ++j) xl[j] = z[j];
+        __syncwarp();
+        rows_out(wt);
+        __syncwarp();
+#pragma unroll
+        for (int j = B; j < W; ++j) xl[j - B] = z[j];
+        __syncwarp();
+        if (xr < W - B) rows_out(wt + B);
+        __syncwarp();  // the next group reads these rows from other lanes of this warp
       }
     }
   }
