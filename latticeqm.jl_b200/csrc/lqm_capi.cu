@@ -384,6 +384,23 @@ void launch_zgemm_dmma(cudaStream_t st, const GemmArgs& g, int batch) {
   zgemm_dmma_kernel<BM, BN, WM, WN, BK, ST><<<grid, nt, smem, st>>>(g);
 }
 
+// kernel<<<cs nk, nt, smem>>>(args...) in clusters of cs blocks
+template <class... P, class... Q>
+void launch_cluster(cudaStream_t st, void (*kernel)(P...), int cs, int64_t nk, int nt, int smem, Q... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)cs;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(cs * nk));
+  cfg.blockDim = dim3((unsigned)nt);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = cs > 1 ? 1 : 0;
+  ck(cudaLaunchKernelEx(&cfg, kernel, P(args)...), "cluster launch");
+}
+
 // C_b = alpha op(A_b) op(B_b) + beta C_b for b < batch (column-major, strided):
 // the library's DMMA kernel (lqm_zgemm.cuh), with the tile shape chosen by the
 // product's shape (skinny n: the Fourier fold; small m: the back-transformation's
@@ -432,14 +449,21 @@ void zgemm_sb(lqm_ctx* ctx, GemmOp ta, GemmOp tb, int m, int n, int k, double al
       return;
     }
   }
-  if (n <= 16 && m >= 512)
-    launch_zgemm_dmma<128, 16, 16, 16, 8, 3>(h, g, batch);  // eight warps per tile: tall skinny products
-  else if (n <= 16)
-    launch_zgemm_dmma<128, 16, 32, 16, 8, 3>(h, g, batch);
+  // Tiles of four warps, 16 x 16 each, four CTAs per SM, where the k-loop is short or one
+  // side is narrow: what these products wait for is the start and the end of a tile, and
+  // four CTAs overlap them better than two of eight warps.  Measured on 64 matrices,
+  // TFLOP/s: the panel product Y = A22 V (n = 16) at m = 1200 / 300: 21.5 / 14.7 on
+  // 64 x 16 tiles against 16.3 / 11.5 on 128 x 16; U -= V Y (k = 64, n = 693) at m = 1200 /
+  // 300: 23.9 / 22.1 on 32 x 32 against 23.3 / 20.7 on 64 x 64 of eight warps.  V^H U
+  // (m = 64) has a long k and keeps 64 x 64, its warps 16 x 32: 28.4 against 24.8 for 32 x 32.
+  if (n <= 16)
+    launch_zgemm_dmma<64, 16, 16, 16, 8, 3>(h, g, batch);
   else if (m <= 32)
     launch_zgemm_dmma<32, 64, 32, 16, 8, 3>(h, g, batch);
   else if (k <= 64)
-    launch_zgemm_dmma<64, 64, 32, 16, 8, 3>(h, g, batch);
+    launch_zgemm_dmma<32, 32, 16, 16, 8, 3>(h, g, batch);
+  else if (m <= 64 && n >= 128)
+    launch_zgemm_dmma<64, 64, 16, 32, 8, 3>(h, g, batch);
   else {
     // the tile that computes least: for orders that are no multiple of 64 the padding of
     // 64 x 64 tiles is most of the work (n = 72: 128 x 128).  The smaller tiles load more
@@ -468,7 +492,13 @@ void zher2k_lower(lqm_ctx* ctx, int m, int k, const double2* X, int ldx, long lo
   if (batch > 65535) fail(LQM_EINVAL, "GEMM batch %d exceeds the grid limit", batch);
   GemmArgs g{m, m, k, -1.0, 1.0, X, ldx, sX, Y, ldy, sY, C, ldc, sC, (int)OP_N, (int)OP_C, 0, k,
              Y, ldy, sY, X, ldx, sX, k, 1};
-  launch_zgemm_dmma<64, 64, 32, 16, 8, 3>(ctx->stream, g, batch);
+  // 16 warps of 16 x 16 on 64 x 64 (the tile is loaded, updated and stored in a burst: half
+  // the time is C itself), 32 x 32 tiles of four warps below 512 rows.  64 matrices, m = 1200:
+  // 0.67 ms against 0.77 with eight warps; m = 300: 0.060 against 0.066 with 64 x 64.
+  if (m >= 512)
+    launch_zgemm_dmma<64, 64, 16, 16, 8, 2>(ctx->stream, g, batch);
+  else
+    launch_zgemm_dmma<32, 32, 16, 16, 8, 3>(ctx->stream, g, batch);
   ck(cudaGetLastError(), "zher2k launch");
 }
 
@@ -531,7 +561,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   const int64_t pstride = ts ? 0 : symv_part_stride(n), tstride = ts ? 0 : t12_part_stride(n, nb);
   const int64_t auxk = 2 * (int64_t)n * wc /*W, Y*/ + (int64_t)nbt * nbt * P2 /*Tm*/ + n /*tau*/ + 2 * nb /*t12*/ +
                        pstride /*mat-vec partials*/ + tstride /*panel-product partials*/;
-  const int64_t tspk = ts ? 3 * (int64_t)n * kTsB + 3 * kTsB * kTsB : 0;   // Vb, Y, X; T, S, Z
+  const int64_t tspk = ts ? 3 * (int64_t)n * kTsB + kTsB * kTsB : 0;   // Vb, Y, W; T
   const int64_t tsbk = ts ? 2 * (int64_t)kTsB * n : 0;                        // the band
   const int64_t tsvk = (ts && vec) ? ts_v2_stride(n) + ts_tau2_stride(n) : 0; // stage-2 reflectors
   const double per_k = 16.0 * (double)nn * ((vec && !d_U) ? 2.0 : 1.0) + 16.0 * (double)(auxk + tspk + tsbk + tsvk) +
@@ -595,21 +625,27 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
       double2* Vb = tsp;                              // nbk x (n x kTsB)
       double2* Yt = Vb + B * (int64_t)n * kTsB;
       double2* Xt = Yt + B * (int64_t)n * kTsB;
-      double2* Tt = Xt + B * (int64_t)n * kTsB;       // nbk x (kTsB x kTsB): T, S, Z
-      double2* St = Tt + B * (int64_t)kTsB * kTsB;
-      double2* Zt = St + B * (int64_t)kTsB * kTsB;
-      const long long sv = (long long)n * kTsB, s2 = (long long)kTsB * kTsB;
+      double2* Tt = Xt + B * (int64_t)n * kTsB;       // nbk x (kTsB x kTsB)
+      const long long sv = (long long)n * kTsB;
+      ck(cudaFuncSetAttribute(ts_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsWSmem), "smem attr");
       for (int j0 = 0; j0 + kTsB < n; j0 += kTsB) {
         const int m = n - j0 - kTsB, nr = std::min(kTsB, m);
-        ts_panel_kernel<<<nbk, kTsPanelThreads, 0, ctx->stream>>>(n, j0, A, tau, Vb, Tt);
+        const int pc = (m + kTsPanelThreads - 1) / kTsPanelThreads;
+        if (pc <= kTsPanelMaxCluster)  // whole warps, the rows shared evenly
+          launch_cluster(ctx->stream, ts_panel_reg_kernel, pc, nbk, ((m + pc - 1) / pc + 31) / 32 * 32, 0, n, j0, pc, A,
+                         tau, Vb, Tt);
+        else
+          ts_panel_kernel<<<nbk, kTsPanelThreads, 0, ctx->stream>>>(n, j0, A, tau, Vb, Tt);
         double2* A22 = A + (j0 + kTsB) + (int64_t)(j0 + kTsB) * n;
-        zgemm_sb(h, OP_HL, OP_N, m, nr, m, 1.0, A22, n, nn, Vb, n, sv, 0.0, Yt, n, sv, nbk);           // Y = A22 V
-        zgemm_sb(h, OP_N, OP_N, m, nr, nr, 1.0, Yt, n, sv, Tt, kTsB, s2, 0.0, Xt, n, sv, nbk);         // X = Y T
-        zgemm_sb(h, OP_C, OP_N, nr, nr, m, 1.0, Vb, n, sv, Xt, n, sv, 0.0, St, kTsB, s2, nbk);         // S = V^H X
-        zgemm_sb(h, OP_C, OP_N, nr, nr, nr, 0.5, Tt, kTsB, s2, St, kTsB, s2, 0.0, Zt, kTsB, s2, nbk);  // Z = T^H S / 2
-        zgemm_sb(h, OP_N, OP_N, m, nr, nr, -1.0, Vb, n, sv, Zt, kTsB, s2, 1.0, Xt, n, sv, nbk);        // W = X - V Z
+        zgemm_sb(h, OP_HL, OP_N, m, nr, m, 1.0, A22, n, nn, Vb, n, sv, 0.0, Yt, n, sv, nbk);  // Y = A22 V
+        // W (into Xt): blocks of at least 128 rows, as many as fill the SMs twice
+        int wc = std::min((m + 127) / 128, std::max(1, 2 * ctx->num_sms / nbk));
+        wc = std::min(wc, kTsWMaxCluster);
+        const int wrows = ((m + wc - 1) / wc + 15) / 16 * 16;
+        launch_cluster(ctx->stream, ts_w_kernel, wc, nbk, kTsWThreads, kTsWSmem, n, m, nr, wc, wrows,
+                       (const double2*)Vb, (const double2*)Yt, (const double2*)Tt, Xt);
         zher2k_lower(h, m, nr, Vb, n, sv, Xt, n, sv, A22, n, nn, nbk);                                 // A22 -= V W^H + W V^H
-        ctx->launches += 7;
+        ctx->launches += 4;
       }
       // stage 2: the band, then the bulge chase to the real tridiagonal
       ts_band_kernel<<<nbk, kBlkThreads, 0, ctx->stream>>>(n, A, Bd);

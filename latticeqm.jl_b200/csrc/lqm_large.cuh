@@ -738,6 +738,275 @@ __global__ void __launch_bounds__(kTsPanelThreads) ts_panel_kernel(int n, int j0
                     Tm + b * kTsB * kTsB, sm);
 }
 
+// ---- cluster helpers (all blocks of a cluster work on one k-point) ----
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// store 16 bytes at the shared-memory address of block `rank` that corresponds to p
+__device__ __forceinline__ void cluster_st16(void* p, int rank, double2 v) {
+  unsigned ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};\n" ::"r"(ra), "d"(v.x), "d"(v.y) : "memory");
+}
+
+// Sums of 16 values over the warp: every lane gets the total of value lane % 16
+// (an exchange tree: 16 shuffles instead of 80).
+__device__ __forceinline__ double warp_sum16(double (&v)[16], int lane) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const bool up = lane & o;
+      const double keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + o], o);
+    }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+// The panel factorisation of ts_panel_qr with the panel in registers: thread = one row of
+// the panel (16 complex), a cluster of cs = ceil(m / 512) blocks per k-point, each with its
+// share of the rows (blockDim.x of them).
+// A column takes one reduction: the sums of conj(x_r) a_l(r) over the rows below the
+// head, for all 16 columns l at once, hold the column's norm, the products with
+// the columns to the right (scaled afterwards, the head row added) and with the finished
+// reflectors to the left, which are the Gram matrix that T is formed from.  One block
+// barrier per column (and one cluster barrier where cs > 1), against five barriers and three
+// passes over global memory in ts_panel_qr.  The registers rotate by a column per step, so
+// that the loop is not unrolled: unrolled, its 16 different steps are fetched from L2 once
+// each and take 91 us at m = 348.  Bound by that chain of 16 steps: 31 us per panel of the
+// n = 364 reduction (32 k-points, average) and 100 of the n = 1324 one (144), against 97 and 165
+// in ts_panel_qr's form.
+constexpr int kTsPanelMaxCluster = 8;  // the portable cluster size; longer panels take ts_panel_kernel
+__global__ void __launch_bounds__(kTsPanelThreads, 1) ts_panel_reg_kernel(int n, int j0, int cs, double2* A,
+                                                                          double2* tau, double2* Vb, double2* Tm) {
+  constexpr int B = kTsB, NW = kTsPanelThreads / 32;
+  static_assert(B == 16, "half a warp holds the sums of the 16 columns");
+  __shared__ __align__(16) double2 part[2][NW][B];               // warp sums
+  __shared__ __align__(16) double2 head[2][B];                   // the head row before its column
+  __shared__ __align__(16) double2 tot[2][kTsPanelMaxCluster][B];  // block sums of the cluster
+  __shared__ __align__(16) double2 wv[NW][B];                    // per warp: conj(tau) w_l
+  __shared__ __align__(16) double2 G[B][B];                      // G[q][l] = v_q^H v_l, q < l
+  __shared__ double2 taus[B];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int rank = blockIdx.x % cs;  // grid (cs nk), clusters of cs consecutive blocks
+  const int64_t b = blockIdx.x / cs;
+  const int m = n - j0 - B, nr = m < B ? m : B;
+  const int r = rank * (int)blockDim.x + tid;  // this thread's row, counted from j0 + B
+  const bool valid = r < m;
+  double2* Ar = A + b * (int64_t)n * n + (int64_t)j0 * n + (j0 + B) + r;  // + l n: column l
+  double2* Vr = Vb + b * (int64_t)n * B + r;
+  double2 a[B];  // slot l: column (c + l) % 16 at step c (the finished ones hold their reflectors)
+#pragma unroll
+  for (int l = 0; l < B; ++l) a[l] = valid ? Ar[(int64_t)l * n] : cmk(0.0, 0.0);
+  for (int e = tid; e < B * B; e += blockDim.x) ((double2*)G)[e] = cmk(0.0, 0.0);
+  if (tid < B) taus[tid] = cmk(0.0, 0.0);
+  if (cs > 1) cluster_barrier();  // every block of the cluster runs before its shared memory is written
+#pragma unroll 1
+  for (int c = 0; c < nr; ++c) {
+    const int par = c & 1;
+    const double2 x = (r > c) ? a[0] : cmk(0.0, 0.0);
+    double t[B];
+#pragma unroll
+    for (int l = 0; l < B; ++l) t[l] = x.x * a[l].x + x.y * a[l].y;
+    const double sr = warp_sum16(t, lane);
+#pragma unroll
+    for (int l = 0; l < B; ++l) t[l] = x.x * a[l].y - x.y * a[l].x;
+    const double si = warp_sum16(t, lane);
+    if (lane < B) part[par][warp][lane] = cmk(sr, si);
+    if (r == c) {
+#pragma unroll
+      for (int l = 0; l < B; ++l) head[par][l] = a[l];
+    }
+    __syncthreads();
+    // lane l (and l + 16): the block's sum of slot l, every second warp in each half
+    const int l0 = lane & 15;
+    double2 v = cmk(0.0, 0.0);
+    if (cs == 1 || warp == 0) {
+#pragma unroll
+      for (int q = 0; q < NW; q += 2)
+        if (q + (lane >> 4) < nw) v = cadd(v, part[par][q + (lane >> 4)][l0]);
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+    }
+    if (cs > 1) {
+      if (warp == 0 && lane < B) {
+        for (int q = 0; q < cs; ++q) cluster_st16(&tot[par][rank][lane], q, v);
+        if (rank == 0)
+          for (int q = 1; q < cs; ++q) cluster_st16(&head[par][lane], q, head[par][lane]);
+      }
+      cluster_barrier();
+      v = cmk(0.0, 0.0);
+      for (int q = 0; q < cs; ++q) v = cadd(v, tot[par][q][l0]);
+    }
+    const double s = __shfl_sync(0xffffffffu, v.x, 0);
+    double2 tj, scal;
+    double beta;
+    zlarfg_scalars(head[par][0], s, &tj, &beta, &scal);
+    const double2 w = cadd(head[par][l0], cmulc(scal, v));  // v_c^H a_l
+    const bool right = l0 > 0 && c + l0 < B;                // a column still to be reduced
+    if (lane < B) wv[warp][lane] = right ? cmul(cconj(tj), w) : cmk(0.0, 0.0);
+    if (rank == 0 && warp == 0 && lane < B && c + lane >= B) G[c + lane - B][c] = cconj(w);
+    if (rank == 0 && tid == 0) { taus[c] = tj; tau[b * n + j0 + c] = tj; }
+    __syncwarp();
+    // column c: R above the head, beta in it, the reflector below; the explicit reflector
+    const double2 vc = (r == c) ? cmk(1.0, 0.0) : cmul(scal, x);
+    if (valid) {
+      Ar[(int64_t)c * n] = (r < c) ? a[0] : (r == c) ? cmk(beta, 0.0) : vc;
+      Vr[(int64_t)c * n] = vc;
+    }
+#pragma unroll
+    for (int l = 0; l + 1 < B; ++l) a[l] = csub(a[l + 1], cmul(vc, wv[warp][l + 1]));
+    a[B - 1] = vc;
+  }
+  if (valid)
+#pragma unroll
+    for (int l = 0; l < B; ++l)
+      if (nr + l < B) Ar[(int64_t)(nr + l) * n] = a[l];
+  // T = (diag(1 / tau) + striu(G))^-1 (zlarft forward), column `lane` by back-substitution:
+  // t_s = -tau_s sum_{i > s} G(s, i) t_i; a zero tau gives a zero row
+  if (rank == 0 && warp == 0) {
+    __syncwarp();
+    double2 acc[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) acc[i] = cmk(0.0, 0.0);
+#pragma unroll
+    for (int s2 = B - 1; s2 >= 0; --s2) {
+      const double2 ts = taus[s2];
+      const double2 tv = (s2 == lane)  ? ts
+                         : (s2 < lane) ? cmul(cmk(-ts.x, -ts.y), acc[s2])
+                                       : cmk(0.0, 0.0);
+#pragma unroll
+      for (int i = 0; i < s2; ++i) acc[i] = cadd(acc[i], cmul(G[i][s2], tv));
+      if (lane < B) Tm[b * B * B + s2 + lane * B] = tv;
+    }
+  }
+}
+
+// W = X - V Z / 2 of the trailing update A22 -= V W^H + W V^H, from V, T and Y = A22 V:
+// X = Y T, Z = T^H V^H X.  With G = V^H Y this is W = Y T - V (T^H G T / 2), one pass over V
+// and Y for G and one for W, tensor steps (DMMA) straight from global memory in both; a
+// cluster of cs blocks per k-point, each with a slice of `rows` rows (a multiple of 16).
+// As five to seven GEMM launches this took 84 us per panel at m = 348.  Bound by latency and,
+// for many k-points, by reading V and Y.
+constexpr int kTsWThreads = 256;
+constexpr int kTsWMaxCluster = 8;
+constexpr int kTsWSmem = (kTsWThreads / 32 + kTsWMaxCluster + 4) * kTsB * kTsB * 16;
+__global__ void __launch_bounds__(kTsWThreads, 2) ts_w_kernel(int n, int m, int nr, int cs, int rows,
+                                                              const double2* V, const double2* Y, const double2* Tm,
+                                                              double2* Wo) {
+  constexpr int B = kTsB, NW = kTsWThreads / 32, BB = B * B;
+  static_assert(BB == kTsWThreads, "a thread per entry of the 16 x 16 products");
+  extern __shared__ __align__(16) unsigned char tsw_smem[];
+  double2* part = (double2*)tsw_smem;        // NW x BB warp sums of G
+  double2* tot = part + NW * BB;             // cs x BB block sums
+  double2* Gm = tot + kTsWMaxCluster * BB;   // G, then S = G T
+  double2* Sm = Gm + BB;
+  double2* Cf = Sm + BB;                     // 32 x 16: T over -Z (row-major)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int rank = blockIdx.x % cs;
+  const int64_t b = blockIdx.x / cs;
+  const double2* Vk = V + b * (int64_t)n * B;
+  const double2* Yk = Y + b * (int64_t)n * B;
+  double2* Wk = Wo + b * (int64_t)n * B;
+  const int rbeg = rank * rows, rend = (rbeg + rows < m) ? rbeg + rows : m;
+  Cf[tid] = Tm[b * BB + (tid / B) + (tid % B) * B];  // Cf[k][l] = T(k, l)
+  if (cs > 1) cluster_barrier();  // every block of the cluster runs before its shared memory is written
+  // G(q, l) = sum_r conj(V(r, q)) Y(r, l)
+  double re[2][2][2], im[2][2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+  for (int r0 = rbeg + 16 * warp; r0 < rend; r0 += 16 * NW) {
+    double2 av[4][2], bv[4][2];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int r = r0 + 4 * kk + t;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const bool ok = r < rend && 8 * i + g < nr;
+        av[kk][i] = ok ? Vk[r + (int64_t)(8 * i + g) * n] : cmk(0.0, 0.0);
+        bv[kk][i] = ok ? Yk[r + (int64_t)(8 * i + g) * n] : cmk(0.0, 0.0);
+      }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          dmma_884(re[i][j][0], re[i][j][1], av[kk][i].x, bv[kk][j].x);
+          dmma_884(re[i][j][0], re[i][j][1], av[kk][i].y, bv[kk][j].y);
+          dmma_884(im[i][j][0], im[i][j][1], av[kk][i].x, bv[kk][j].y);
+          dmma_884(im[i][j][0], im[i][j][1], -av[kk][i].y, bv[kk][j].x);
+        }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        part[warp * BB + (8 * i + g) * B + 8 * j + 2 * t + h] = cmk(re[i][j][h], im[i][j][h]);
+  __syncthreads();
+  double2 sum = part[tid];
+#pragma unroll
+  for (int w = 1; w < NW; ++w) sum = cadd(sum, part[w * BB + tid]);
+  if (cs > 1) {
+    for (int q = 0; q < cs; ++q) cluster_st16(tot + rank * BB + tid, q, sum);
+    cluster_barrier();
+    sum = tot[tid];
+    for (int q = 1; q < cs; ++q) sum = cadd(sum, tot[q * BB + tid]);
+  }
+  Gm[tid] = sum;
+  __syncthreads();
+  const int q = tid / B, l = tid % B;
+  double2 acc = cmk(0.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < B; ++k) acc = cadd(acc, cmul(Gm[q * B + k], Cf[k * B + l]));
+  Sm[tid] = acc;
+  __syncthreads();
+  acc = cmk(0.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < B; ++k) acc = cadd(acc, cmulc(Cf[k * B + q], Sm[k * B + l]));
+  Cf[BB + tid] = cmk(-0.5 * acc.x, -0.5 * acc.y);
+  __syncthreads();
+  // W = [Y V] Cf: the coefficients stay in registers as B fragments
+  double2 bf[8][2];
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) bf[k][j] = Cf[(4 * k + t) * B + 8 * j + g];
+  for (int r0 = rbeg + 8 * warp; r0 < rend; r0 += 8 * NW) {
+    const int r = r0 + g;
+    double2 av[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int cc = 4 * (k & 3) + t;
+      const double2* src = (k < 4) ? Yk : Vk;
+      av[k] = (r < rend && cc < nr) ? src[r + (int64_t)cc * n] : cmk(0.0, 0.0);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        dmma_884(wr[0], wr[1], av[k].x, bf[k][j].x);
+        dmma_884(wr[0], wr[1], -av[k].y, bf[k][j].y);
+        dmma_884(wi[0], wi[1], av[k].x, bf[k][j].y);
+        dmma_884(wi[0], wi[1], av[k].y, bf[k][j].x);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int cc = 8 * j + 2 * t + h;
+        if (r < rend && cc < nr) Wk[r + (int64_t)cc * n] = cmk(wr[h], wi[h]);
+      }
+    }
+  }
+}
+
 // grid (B): the band (2 kTsB x n per k-point) out of the stage-1 result.
 __global__ void __launch_bounds__(kBlkThreads) ts_band_kernel(int n, const double2* A, double2* Bd) {
   const Team T = make_team();

@@ -1,0 +1,43 @@
+"""The two-stage eigensolver at the edges of its panels, their blocks and the column blocks
+of its back-transformation."""
+import numpy as np
+import pytest
+
+from oracle import kspace as K
+from test_gpu_odd_orders import vacancy_cell
+
+pytestmark = pytest.mark.gpu
+BAND_TOL = 1e-10  # of the spectral width, as in test_gpu_parity
+RHO_TOL = 1e-9
+
+# bands of 16: one row below the first panel (18), short last panels (31 .. 49); column
+# blocks of 128 (144, 145); panels of 512 rows in one block and of 513 and more in
+# two (528, 529), of 1025 in three (1041)
+ORDERS = [18, 31, 32, 33, 48, 49, 144, 145, 528, 529, 1041]
+
+
+@pytest.mark.parametrize("n", ORDERS)
+def test_two_stage_matches_oracle(lqm, n):
+    c = lqm.Context()
+    c.set_blocked_min_n(1)
+    c.set_two_stage(1)
+    nk = 3 if n < 500 else 2
+    h = vacancy_cell(n, seed=n)
+    ks = np.random.default_rng(n).uniform(-0.5, 0.5, (2, nk))
+    b, U = lqm.bandmatrix(h, ks, want_vectors=True, ctx=c)
+    ref, _ = K.bandmatrix(h, ks)
+    width = np.ptp(ref)
+    assert np.max(np.abs(b - ref)) <= BAND_TOL * width
+    assert np.max(np.abs(lqm.bandmatrix(h, ks, ctx=c)[0] - ref)) <= BAND_TOL * width
+    for j in range(nk):
+        Hk = K.fouriersum(h, ks[:, j])
+        assert np.max(np.abs(Hk @ U[:, :, j] - U[:, :, j] * b[:, j])) <= BAND_TOL * width
+        assert np.max(np.abs(U[:, :, j].conj().T @ U[:, :, j] - np.eye(n))) <= 1e-12 * max(1.0, n / 144)
+    w = np.full(nk, 1.0 / nk)
+    for mu in (0.0, 0.4 * ref.max()):  # half and nearly all states full
+        rho = {R: None for R in h}
+        e = lqm.getdensitymatrix(rho, h, ks, mu=mu, T=0.01, ctx=c)
+        rref, eref = K.densitymatrix(h, ks, w, mu, 0.01, list(h.keys()))
+        assert max(np.max(np.abs(rho[R] - rref[R])) for R in h) <= RHO_TOL
+        assert abs(e - eref) <= 1e-9 * max(1.0, n * width)
+    c.close()
