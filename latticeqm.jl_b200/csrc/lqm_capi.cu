@@ -616,9 +616,9 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   if (ctx->stats_on) { evs = stat_events(ctx); ck(cudaEventRecord(evs.first, ctx->stream), "event"); }
   for (int64_t k0 = 0; k0 < nk; k0 += B) {
     const int nbk = (int)std::min<int64_t>(B, nk - k0);
-    const size_t bsm = (size_t)H->nR * sizeof(double2) + (size_t)H->d * sizeof(double) + 16;
-    blk_bloch_kernel<<<nbk, kBlkThreads, bsm, ctx->stream>>>(n, (int)H->nR, H->d, H->blocks, H->keys, nbk,
-                                                              d_ks + k0 * H->d, A);
+    const int64_t bt = (n + 31) / 32;
+    blk_bloch_kernel<<<(unsigned)(bt * (bt + 1) / 2 * ((nbk + kBlochK - 1) / kBlochK)), kBlkThreads, 0, ctx->stream>>>(
+        n, (int)H->nR, H->d, H->blocks, H->keys, nbk, d_ks + k0 * H->d, A);
     ctx->launches++;
     if (ts) {
       // stage 1: per panel the QR below the band, then A22 <- Q^H A22 Q by GEMMs
