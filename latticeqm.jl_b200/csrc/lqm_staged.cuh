@@ -880,7 +880,7 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
         const double rho = S.nrho[q], di = dl[it];
         for (int j = t; j < kk; j += 4) {
           const double dij = (di - dl[S.org[lo + j]]) - S.troot[lo + j];
-          prod *= -dij / (j == it ? rho : dl[j] - di);
+          prod *= lqm_div_normal(-dij, j == it ? rho : dl[j] - di);
         }
       }
       prod *= __shfl_xor_sync(FULL, prod, 1);
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
           const double lorg = dl[S.org[c]], tq = S.troot[c];
           double ss = 0.0, f = 0.0, l = 0.0;
           for (int p = lane; p < kk; p += 32) {
-            const double u = S.zhat[lo + p] / ((dl[p] - lorg) - tq);
+            const double u = lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq);
             const int col = S.colnd[lo + p];
             ss += u * u;
             f += FT[col] * u;
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
       for (int x = 0; x < kk; x += 4) {
         const bool px = x + t < kk;
         const int p = px ? pl[lo + x + t] : 0, col = px ? pq[lo + x + t] : lo;
-        const double u = (in && px) ? S.zhat[lo + p] / ((dl[p] - lorg) - tq) : 0.0;
+        const double u = (in && px) ? lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq) : 0.0;
         ss = fma(u, u, ss);
         const double* qc = Q + (size_t)col * n;
         const bool upper = x < kum, lower = x + 4 > ku;  // uniform
