@@ -275,7 +275,7 @@ enum WsSlot {
   WS_SCRATCH = 0, WS_KS, WS_BANDS, WS_U, WS_RHOK, WS_COEF, WS_EBK, WS_RHO, WS_W, WS_MISC, WS_PART,
   WS_OMEGA, WS_DOS, WS_LKEYS, WS_HF, WS_HF2, WS_MU, WS_BANDS2,
   WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_VU, WS_VB, WS_VX, WS_VT, WS_VG, WS_ONES, WS_SCFY, WS_AND, WS_EXCH, WS_HFPART, WS_BDG, WS_BDGE, WS_BDGI, WS_BDGK, WS_BDGP, WS_BDGB, WS_CSC, WS_UNIW, WS_SPAN, WS_GRAD, WS_GRADE, WS_HFPART2, WS_GEMMSPLIT, WS_GRAM, WS_TSP, WS_TSB, WS_TSV2,
-  WS_STV, WS_STZ, WS_STU, WS_STI, WS_STOCC
+  WS_STV, WS_STZ, WS_STU, WS_STI, WS_STOCC, WS_LDCQ, WS_LDCREC
 };
 static_assert(WS_STOCC < 64, "workspace slots");
 
@@ -564,7 +564,9 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   const int64_t tspk = ts ? 3 * (int64_t)n * kTsB + kTsB * kTsB : 0;   // Vb, Y, W; T
   const int64_t tsbk = ts ? 2 * (int64_t)kTsB * n : 0;                        // the band
   const int64_t tsvk = (ts && vec) ? ts_v2_stride(n) + ts_tau2_stride(n) : 0; // stage-2 reflectors
-  const double per_k = 16.0 * (double)nn * ((vec && !d_U) ? 2.0 : 1.0) + 16.0 * (double)(auxk + tspk + tsbk + tsvk) +
+  const bool root = vec && n >= kDcTileMin;  // the last merge forms its vectors in dc_root_kernel
+  const int root_mid = n / 2;
+  const double per_k = 16.0 * (double)nn * ((vec && !d_U) ? 2.0 : 1.0) + (root ? 8.0 * (double)nn : 0.0) + 16.0 * (double)(auxk + tspk + tsbk + tsvk) +
                        16.0 * n;
   int64_t B = std::max<int64_t>(1, std::min<int64_t>(nk, (int64_t)(64.0e9 / per_k)));
   B = std::min<int64_t>(B, 65535);
@@ -592,6 +594,9 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   double2* V2 = (ts && vec) ? (double2*)ws_get(ctx, WS_TSV2, (size_t)B * tsvk * sizeof(double2)) : nullptr;
   double2* tau2 = V2 ? V2 + B * ts_v2_stride(n) : nullptr;
   double* slots = (double*)ws_get(ctx, WS_LDC, (size_t)G * slotd * sizeof(double));
+  // the last merge's vectors by a kernel of its own (from the order on that has tiled merges)
+  double* rootQ = root ? (double*)ws_get(ctx, WS_LDCQ, (size_t)(B * nn) * sizeof(double)) : nullptr;
+  double* rootRec = root ? (double*)ws_get(ctx, WS_LDCREC, (size_t)(B * dc_root_rec_doubles(n)) * sizeof(double)) : nullptr;
   const DCPlan& plan = get_plan(ctx, n);
   lqm_ctx* h = blas_handle(ctx);
   CUtensorMap symv_map, symv_vmap;
@@ -711,6 +716,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
     da.n = n; da.nk = nbk; da.plan = plan; da.d = dd; da.e = ee; da.bands = d_bands + k0 * n;
     da.U = vec ? Ucur : nullptr; da.slots = slots; da.slot_doubles = slotd;
     da.phase_cycles = ctx->phases_on ? ctx->d_phase : nullptr;
+    da.Qk = rootQ; da.rec = rootRec;
     if (dc_small)
       dc_large_kernel<128, 4><<<(unsigned)std::min<int64_t>(G, nbk), 128, 0, ctx->stream>>>(da);
     else
@@ -739,6 +745,12 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
       } else {
         K = hspan[1];
       }
+    }
+    if (K > 0 && root) {
+      ck(cudaFuncSetAttribute(dc_root_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDcRootSmem), "smem attr");
+      const dim3 rg((unsigned)((K + 63) / 64), (unsigned)dc_root_row_tiles(n, root_mid), (unsigned)nbk);
+      dc_root_kernel<<<rg, kDcRootThreads, kDcRootSmem, ctx->stream>>>(n, root_mid, c0, K, rootQ, rootRec, Ucur);
+      ctx->launches++;
     }
     if (K > 0 && ts) {
       // Z <- Q2 Z on the K columns: the stage-2 reflectors in groups of 16 sweeps,

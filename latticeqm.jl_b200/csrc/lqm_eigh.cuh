@@ -447,8 +447,12 @@ LQM_FN void deflate_node(int node, const DCPlan& P, EighVec& S, double eabs_beta
 #endif
 
 // Merge update of one node as a tiled GEMM (large merges):
-//   Qt[lo + r, newpos[it]] = sum_p Q[lo + r, colnd[p]] * Ubn[it + p*k],
-// r < hi - lo, it < k (Ubn holds the secular vectors as rows).  A 512-thread
+//   Qt[lo + r, newpos[it]] = sum_p Q[lo + r, colnd[ord[p]]] * Ubn[it + p*k],
+// r < hi - lo, it < k (Ubn holds the secular vectors as rows).  The columns are ordered
+// (ord) by the child they come from: [0, nu) upper child only, [nu, nm) both (rotated
+// together), [nm, k) lower child only.  An upper column is zero in the lower child's rows and
+// the other way round, so the rows below mid sum over [0, nm) and the others over [nu, k): half
+// the products.  A 512-thread
 // team computes 128 x 128 output tiles on the FP64 tensor path (DMMA
 // m8n8k4): 16 warps of 32 x 32, each a 4 x 4 grid of 8 x 8 accumulators.  The
 // p range moves in 16-deep stages by cp.async through a 3-stage ring in `tile`
@@ -457,7 +461,7 @@ LQM_FN void deflate_node(int node, const DCPlan& P, EighVec& S, double eabs_beta
 // pairs), followed by room for k column indices; two stages are in flight while
 // one is summed.  p is summed in ascending 4-deep steps.  Other team sizes (the
 // host emulation) take the plain loop.
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDACC__)
 __device__ __forceinline__ void lqm_cp_async8(void* sdst, const void* gsrc, bool valid) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
   const int nbytes = valid ? 8 : 0;  // 0: zero-filled, nothing is read
@@ -469,9 +473,9 @@ constexpr int kDcTileBK = 16;                            // p depth of a stage
 constexpr int kDcTileStage = kDcTileBK * 2 * kDcTileP;   // doubles per stage (Q and Ubn slices)
 constexpr int kDcTileRing = 3 * kDcTileStage;            // doubles of the ring
 template <class TeamT>
-LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int hi, int k, const int* colnd, const int* newpos,
+LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int mid, int hi, int k, int nu, int nm, const int* colnd,
+                         const int* ord, const int* newpos,
                          const double* Q, double* Qt, const double* Ubn, double* tile) {
-  const int s = hi - lo;
 #if defined(__CUDA_ARCH__)
   if (T.nt == 512 && tile != nullptr) {
     constexpr int BM = 128, BN = 128, BK = kDcTileBK, PT = kDcTileP, STG = kDcTileStage, NS = 3;
@@ -479,9 +483,13 @@ LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int hi, int k, const int
     const int g = lane >> 2, t = lane & 3;
     const int wr = (warp & 3) * 32, wc = (warp >> 2) * 32;  // the warp's 32 x 32 sub-tile
     int* cidx = (int*)(tile + kDcTileRing);                  // the node's column indices, staged once
-    for (int p = T.tid; p < k; p += T.nt) cidx[p] = colnd[p];
+    for (int p = T.tid; p < k; p += T.nt) cidx[p] = colnd[ord[p]];
     team_sync(T);
-    for (int r0 = 0; r0 < s; r0 += BM) {
+    const int su = mid - lo, tu = (su + BM - 1) / BM, tl = (hi - mid + BM - 1) / BM;  // row tiles of the two children
+    for (int rt = 0; rt < tu + tl; ++rt) {
+      const int r0 = rt < tu ? rt * BM : su + (rt - tu) * BM;  // first row and end of the tile's child
+      const int s = rt < tu ? su : hi - lo;
+      const int pb = rt < tu ? 0 : nu, pe = rt < tu ? nm : k;
       for (int c0 = 0; c0 < k; c0 += BN) {
         double acc[4][4][2];
 #pragma unroll
@@ -497,21 +505,21 @@ LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int hi, int k, const int
             const int e = T.tid + 512 * h;
             const int pp = e >> 7, x = e & 127;
             const int p = p0 + pp, r = r0 + x, cc = c0 + x;
-            const bool oka = p < k && r < s, okb = p < k && cc < k;
+            const bool oka = p < pe && r < s, okb = p < pe && cc < k;
             lqm_cp_async8(As + pp * PT + x, oka ? (const void*)(Q + (lo + r) + (int64_t)cidx[p] * n) : (const void*)Q,
                           oka);
             lqm_cp_async8(Bs + pp * PT + x, okb ? (const void*)(Ubn + cc + (int64_t)p * k) : (const void*)Ubn, okb);
           }
         };
-        const int nst = (k + BK - 1) / BK;
-        issue(0, 0);
+        const int nst = (pe - pb + BK - 1) / BK;
+        issue(pb, 0);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-        if (nst > 1) issue(BK, 1);
+        if (nst > 1) issue(pb + BK, 1);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         for (int it = 0; it < nst; ++it) {
           asm volatile("cp.async.wait_group 1;\n" ::: "memory");
           team_sync(T);
-          if (it + 2 < nst) issue((it + 2) * BK, (it + 2) % NS);
+          if (it + 2 < nst) issue(pb + (it + 2) * BK, (it + 2) % NS);
           asm volatile("cp.async.commit_group;\n" ::: "memory");
           const double* As = tile + (it % NS) * STG;
           const double* Bs = As + BK * PT;
@@ -550,13 +558,23 @@ LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int hi, int k, const int
 #endif
   for (int it = T.wid; it < k; it += T.nw) {
     double* dst = Qt + (int64_t)newpos[it] * n;
-    for (int r = T.lane; r < s; r += T.nl) {
+    for (int r = lo + T.lane; r < hi; r += T.nl) {
       double acc = 0.0;
-      for (int p = 0; p < k; ++p) acc += Q[(lo + r) + (int64_t)colnd[p] * n] * Ubn[it + (int64_t)p * k];
-      dst[lo + r] = acc;
+      const int pb = r < mid ? 0 : nu, pe = r < mid ? nm : k;
+      for (int p = pb; p < pe; ++p) acc += Q[r + (int64_t)colnd[ord[p]] * n] * Ubn[it + (int64_t)p * k];
+      dst[r] = acc;
     }
   }
 }
+
+// What the last merge of a matrix leaves to a kernel of its own (dc_root_kernel): the merge's
+// poles in the order of dc_tile_gemm (zh: the secular z, dl: the pole, cidx: its column of Q),
+// and per column of the result, by its final place, the eigenvalue (dl[org] = lorg, tq) with the
+// vector's scale sc, or the column of Q that it is (src >= 0).  hdr: k, nu, nm, mid.
+struct DCRootRec {
+  double *zh, *dl, *lorg, *tq, *sc;
+  int *cidx, *src, *hdr;
+};
 
 // vec == false: eigenvalues only.  The merges then need just the first and
 // last rows of each node's eigenvector matrix (they form z), so Q (>= 4n
@@ -568,7 +586,7 @@ LQM_FN void dc_tile_gemm(const TeamT& T, int n, int lo, int hi, int k, const int
 template <class TeamT>
 LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S, double* Q, double* Qt,
                               unsigned long long* sub = nullptr, bool vec = true, double* Ub = nullptr,
-                              int tile_min = 1 << 30) {
+                              int tile_min = 1 << 30, const DCRootRec* root = nullptr) {
   double* ubuf = (double*)S.pbuf;  // per-warp secular eigenvectors (2n doubles each)
   double* QF = Q;
   double* QL = Q + n;
@@ -784,35 +802,89 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
     bool tiled = false;
     if (vec && Ub != nullptr)
       for (int nd = h0; nd < h1; ++nd) tiled = tiled || (P.hi[nd] - P.lo[nd] >= tile_min);
+    const bool defer = tiled && root != nullptr && h == P.nheights - 1;  // one node, the whole matrix
     if (tiled) {
-      // secular vectors into Ub (warp per column), deflated columns copied
+      // the child that each column comes from (1 upper, 2 lower, 3 both after a rotation) in
+      // S.z, then the order of the poles by it in S.perm and its limits in S.nrot, S.ndef
+      for (int i = T.tid; i < n; i += T.nt)
+        if (own[i] >= 0) S.z[i] = (i < P.mid[own[i]]) ? 1.0 : 2.0;
+      team_sync(T);
+      for (int nd = h0 + T.tid; nd < h1; nd += T.nt) {
+        const int lo = P.lo[nd], k = S.nk[nd], nr = S.nrot[nd];
+        for (int t = 0; t < nr; ++t) {
+          const int a = S.ri[lo + t], b = S.rj[lo + t];
+          if (S.z[a] != S.z[b]) S.z[a] = S.z[b] = 3.0;
+        }
+        int c = 0;
+        for (int p = 0; p < k; ++p)
+          if (S.z[S.colnd[lo + p]] == 1.0) S.perm[lo + c++] = p;
+        S.nrot[nd] = c;
+        for (int p = 0; p < k; ++p)
+          if (S.z[S.colnd[lo + p]] == 3.0) S.perm[lo + c++] = p;
+        S.ndef[nd] = c;
+        for (int p = 0; p < k; ++p)
+          if (S.z[S.colnd[lo + p]] == 2.0) S.perm[lo + c++] = p;
+      }
+      // each column's eigenvalue origin (S.rs) and scale (S.rc); deflated columns are copied
       for (int c = T.wid; c < n; c += T.nw) {
         const int nd = own[c];
         if (nd < 0) continue;
         const int lo = P.lo[nd], hi = P.hi[nd], it = c - lo, k = S.nk[nd];
         if (it < k) {
-          double* ub = Ub + (int64_t)lo * n + it;  // row it of the node's k x k block (stride k)
           const double* dl = S.dl + lo;
           const double lorg = dl[S.org[lo + it]], tq = S.troot[lo + it];
           double ss = 0.0;
           for (int p = T.lane; p < k; p += T.nl) {
             const double u = lqm_div_normal(S.zhat[lo + p], (dl[p] - lorg) - tq);
-            ub[(int64_t)p * k] = u;
             ss += u * u;
           }
-          const double sc = 1.0 / sqrt(warp_sum_bcast(ss));
-          for (int p = T.lane; p < k; p += T.nl) ub[(int64_t)p * k] *= sc;
-        } else {
+          ss = warp_sum_bcast(ss);
+          if (T.lane == 0) { S.rc[c] = 1.0 / sqrt(ss); S.rs[c] = lorg; }
+        } else if (!defer) {
           double* dst = Qt + (int64_t)S.newpos[c] * n;
           const double* src = Q + (int64_t)S.dcol[lo + it - k] * n;
           for (int r = lo + T.lane; r < hi; r += T.nl) dst[r] = src[r];
         }
       }
       team_sync(T);
+    }
+    if (defer) {
+      const int k = S.nk[h0];
+      for (int i = T.tid; i < n; i += T.nt) {
+        const int c = S.newpos[i];
+        if (i < k) {
+          const int o = S.perm[i];
+          root->zh[i] = S.zhat[o]; root->dl[i] = S.dl[o]; root->cidx[i] = S.colnd[o];
+          root->lorg[c] = S.rs[i]; root->tq[c] = S.troot[i]; root->sc[c] = S.rc[i];
+          root->src[c] = -1;
+        } else {
+          root->src[c] = S.dcol[i - k];
+        }
+      }
+      if (T.tid == 0) { root->hdr[0] = k; root->hdr[1] = S.nrot[h0]; root->hdr[2] = S.ndef[h0]; root->hdr[3] = P.mid[h0]; }
+    } else if (tiled) {
+      // the secular vectors into Ub, row p of the k x k block by lanes over the columns
+      for (int nd = h0; nd < h1; ++nd) {
+        const int lo = P.lo[nd], k = S.nk[nd];
+        double* ub = Ub + (int64_t)lo * n;
+        const int nc = (k + T.nl - 1) / T.nl;
+        for (int w = T.wid; w < 2 * nc; w += T.nw) {  // chunks of columns, two halves of the rows
+          const int it = (w >> 1) * T.nl + T.lane;
+          if (it >= k) continue;
+          const double lorg = S.rs[lo + it], tq = S.troot[lo + it], sc = S.rc[lo + it];
+          const int pe = (w & 1) ? k : k / 2;
+#pragma unroll 4
+          for (int p = (w & 1) ? k / 2 : 0; p < pe; ++p) {
+            const int o = S.perm[lo + p];
+            ub[it + (int64_t)p * k] = lqm_div_normal(S.zhat[lo + o], (S.dl[lo + o] - lorg) - tq) * sc;
+          }
+        }
+      }
+      team_sync(T);
       for (int nd = h0; nd < h1; ++nd) {
         const int lo = P.lo[nd];
-        dc_tile_gemm(T, n, lo, P.hi[nd], S.nk[nd], S.colnd + lo, S.newpos + lo, Q, Qt, Ub + (int64_t)lo * n,
-                     S.tile);
+        dc_tile_gemm(T, n, lo, P.mid[nd], P.hi[nd], S.nk[nd], S.nrot[nd], S.ndef[nd], S.colnd + lo, S.perm + lo,
+                     S.newpos + lo, Q, Qt, Ub + (int64_t)lo * n, S.tile);
       }
     }
     // Columns in pairs (2t, 2t+1) by warp: when both are non-deflated columns
@@ -904,7 +976,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
     team_sync(T);
     LQM_SUBTICK(6);
     // I: write back
-    for (int c = T.wid; c < n && vec; c += T.nw) {
+    for (int c = T.wid; c < n && vec && !defer; c += T.nw) {
       const int nd = own[c];
       if (nd < 0) continue;
       const int lo = P.lo[nd], hi = P.hi[nd];

@@ -598,7 +598,18 @@ struct DCLargeArgs {
   double* slots;     // gridDim.x slots
   int64_t slot_doubles;
   unsigned long long* phase_cycles;  // [16] as eigh_kernel's (d&c total and merge steps), or null
+  double* Qk;        // nk x (n x n): the vectors before the last merge, left to dc_root_kernel with
+  double* rec;       // nk x dc_root_rec_doubles(n); or null (U is written here)
 };
+
+// doubles of one k-point's record of its last merge (DCRootRec)
+__host__ __device__ inline int64_t dc_root_rec_doubles(int n) { return 5 * (int64_t)n + (2 * (int64_t)n + 4 + 1) / 2; }
+__host__ __device__ inline DCRootRec dc_root_rec(double* p, int n) {
+  DCRootRec r;
+  r.zh = p; r.dl = p + n; r.lorg = p + 2 * (int64_t)n; r.tq = p + 3 * (int64_t)n; r.sc = p + 4 * (int64_t)n;
+  r.cidx = (int*)(p + 5 * (int64_t)n); r.src = r.cidx + n; r.hdr = r.src + n;
+  return r;
+}
 
 __host__ __device__ inline int64_t dc_large_slot_doubles(int n, bool vec) {
   const int64_t nn = (int64_t)n * n;
@@ -637,6 +648,7 @@ __global__ void __launch_bounds__(NT, MINB) dc_large_kernel(DCLargeArgs a) {
   S.pbuf = (double2*)(((uintptr_t)pb + 15) & ~(uintptr_t)15);
   S.tau = S.v = S.w = S.vn = S.pn = S.bc = nullptr;
   S.tile = tile;
+  DCRootRec rec;
   const bool prof = a.phase_cycles != nullptr;
   unsigned long long dsub[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   unsigned long long dtot = 0;
@@ -647,10 +659,14 @@ __global__ void __launch_bounds__(NT, MINB) dc_large_kernel(DCLargeArgs a) {
     }
     team_sync();
     const long long t0 = prof ? clock64() : 0;
-    dc_solve(T, n, a.plan, S, Q, Qt, prof ? dsub : nullptr, vec, Ub, kDcTileMin);
+    if (a.Qk) {
+      Q = a.Qk + k * nn;
+      rec = dc_root_rec(a.rec + k * dc_root_rec_doubles(n), n);
+    }
+    dc_solve(T, n, a.plan, S, Q, Qt, prof ? dsub : nullptr, vec, Ub, kDcTileMin, a.Qk ? &rec : nullptr);
     if (prof) dtot += (unsigned long long)(clock64() - t0);
     for (int i = T.tid; i < n; i += T.nt) a.bands[k * n + i] = S.D[i];
-    if (vec) {
+    if (vec && !a.Qk) {
       double2* Uk = a.U + k * nn;
       for (int c = T.wid; c < n; c += T.nw)
         for (int r = T.lane; r < n; r += T.nl) Uk[r + (int64_t)c * n] = cmk(Q[r + (int64_t)c * n], 0.0);
@@ -661,6 +677,103 @@ __global__ void __launch_bounds__(NT, MINB) dc_large_kernel(DCLargeArgs a) {
     atomicAdd(&a.phase_cycles[PH_DC], dtot);
     for (int i = 0; i < 8; ++i) atomicAdd(&a.phase_cycles[PH_DCSUB + i], dsub[i]);
   }
+}
+
+// The last merge of every k-point: columns c0 .. c0 + K - 1 of its eigenvectors, as complex
+// numbers, from the vectors before it (Q) and its record.  The work of dc_tile_gemm (same order
+// of the poles, each child's rows over its own and the shared ones), but over all SMs however few the k-points are,
+// only for the wanted columns, and with the secular vectors formed as the B tile is
+// staged.  grid (ceil(K / 64), row tiles of both children, nk): 128 x 64 tiles, eight warps of
+// 32 x 32, a ring of three 16-deep stages.  Three quarters of all merge products are this one.
+constexpr int kDcRootThreads = 256;
+constexpr int kDcRootPA = 132, kDcRootPB = 68;  // pitches == 4 mod 16: conflict-free fragment reads
+constexpr int kDcRootStage = 16 * (kDcRootPA + kDcRootPB);
+constexpr int kDcRootSmem = 3 * kDcRootStage * 8;
+__host__ __device__ inline int dc_root_row_tiles(int n, int mid) { return (mid + 127) / 128 + (n - mid + 127) / 128; }
+__global__ void __launch_bounds__(kDcRootThreads, 2) dc_root_kernel(int n, int mid, int c0, int K, const double* Qk,
+                                                                    const double* recs, double2* U) {
+  extern __shared__ __align__(16) double rtile[];
+  constexpr int BK = 16, PA = kDcRootPA, PB = kDcRootPB;
+  const int64_t b = blockIdx.z;
+  const DCRootRec rec = dc_root_rec((double*)recs + b * dc_root_rec_doubles(n), n);
+  const double* Q = Qk + b * (int64_t)n * n;
+  double2* Uk = U + b * (int64_t)n * n;
+  const int k = rec.hdr[0], nu = rec.hdr[1], nm = rec.hdr[2];
+  const int tu = (mid + 127) / 128, rt = blockIdx.y;
+  const int r0 = rt < tu ? rt * 128 : mid + (rt - tu) * 128;
+  const int rend = rt < tu ? mid : n;
+  const int pb = rt < tu ? 0 : nu, pe = rt < tu ? nm : k;
+  const int cb = c0 + blockIdx.x * 64, cend = c0 + K;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int wr = (warp & 3) * 32, wc = (warp >> 2) * 32;
+  // B: thread's column of the tile (fixed) and rows tid / 64 + 4 h of a stage
+  const int bc = cb + (tid & 63);
+  const bool bok = bc < cend && rec.src[bc] < 0;
+  const double lorg = bok ? rec.lorg[bc] : 0.0, tq = bok ? rec.tq[bc] : 0.0, sc = bok ? rec.sc[bc] : 0.0;
+  auto stage_a = [&](int p0, int st) {
+    double* As = rtile + st * kDcRootStage;
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+      const int pp = (tid >> 7) + 2 * h, x = tid & 127, p = p0 + pp, r = r0 + x;
+      const bool ok = p < pe && r < rend;
+      lqm_cp_async8(As + pp * PA + x, ok ? (const void*)(Q + r + (int64_t)rec.cidx[p] * n) : (const void*)Q, ok);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto stage_b = [&](int p0, int st) {
+    double* Bs = rtile + st * kDcRootStage + 16 * PA;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int pp = (tid >> 6) + 4 * h, p = p0 + pp;
+      double u = 0.0;
+      if (bok && p < pe) u = lqm_div_normal(rec.zh[p], (rec.dl[p] - lorg) - tq) * sc;
+      Bs[pp * PB + (tid & 63)] = u;
+    }
+  };
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nst = (pe - pb + BK - 1) / BK;
+  stage_a(pb, 0);
+  stage_a(pb + BK, 1);
+  stage_b(pb, 0);
+  for (int it = 0; it < nst; ++it) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // stage it is in place; stages it + 1 (B) and it + 2 (A) are free to be filled
+    stage_a(pb + (it + 2) * BK, (it + 2) % 3);
+    if (it + 1 < nst) stage_b(pb + (it + 1) * BK, (it + 1) % 3);
+    const double* As = rtile + (it % 3) * kDcRootStage;
+    const double* Bs = As + 16 * PA;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+      double av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) av[i] = As[(kk + t) * PA + wr + 8 * i + g];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bv[j] = Bs[(kk + t) * PB + wc + 8 * j + g];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma_884(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = cb + wc + 8 * j + 2 * t + h;
+      if (c >= cend) continue;
+      const int src = rec.src[c];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + wr + 8 * i + g;
+        if (r < rend) Uk[r + (int64_t)c * n] = cmk(src < 0 ? acc[i][j][h] : Q[r + (int64_t)src * n], 0.0);
+      }
+    }
 }
 
 // Y[k] = U[k] diag(f(eps - mu)) and eband_k = w_k sum_j f_j eps_j; CTA per k.

@@ -12,8 +12,9 @@ RHO_TOL = 1e-9
 
 # bands of 16: one row below the first panel (18), short last panels (31 .. 49); column
 # blocks of 128 (144, 145); panels of 512 rows in one block and of 513 and more in
-# two (528, 529), of 1025 in three (1041)
-ORDERS = [18, 31, 32, 33, 48, 49, 144, 145, 528, 529, 1041]
+# two (528, 529), of 1025 in three (1041); the last merge in a kernel of its own from 160 on,
+# its row tiles of 128 per child and column tiles of 64 (160, 161, 256, 257, 385)
+ORDERS = [18, 31, 32, 33, 48, 49, 144, 145, 160, 161, 256, 257, 385, 528, 529, 1041]
 
 
 @pytest.mark.parametrize("n", ORDERS)
@@ -41,3 +42,26 @@ def test_two_stage_matches_oracle(lqm, n):
         assert max(np.max(np.abs(rho[R] - rref[R])) for R in h) <= RHO_TOL
         assert abs(e - eref) <= 1e-9 * max(1.0, n * width)
     c.close()
+
+
+@pytest.mark.parametrize("levels", [1, 2, 7, 150])
+def test_merges_with_degenerate_levels(lqm, levels):
+    """A 300 x 300 matrix with `levels` distinct eigenvalues: merges that deflate nearly
+    everything or everything, with rotations between columns of both children."""
+    n = 300
+    rng = np.random.default_rng(levels)
+    q, _ = np.linalg.qr(rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))
+    d = np.sort(np.linspace(-1.0, 1.0, levels)[rng.integers(0, levels, n)])
+    H = (q * d) @ q.conj().T
+    h = {(0, 0): 0.5 * (H + H.conj().T)}
+    ks = np.zeros((2, 2))
+    for mode in (1, 0):
+        c = lqm.Context()
+        c.set_blocked_min_n(1)
+        c.set_two_stage(mode)
+        b, U = lqm.bandmatrix(h, ks, want_vectors=True, ctx=c)
+        assert np.max(np.abs(b[:, 0] - d)) <= 1e-12
+        for j in range(2):
+            assert np.max(np.abs(h[(0, 0)] @ U[:, :, j] - U[:, :, j] * b[:, j])) <= 1e-12
+            assert np.max(np.abs(U[:, :, j].conj().T @ U[:, :, j] - np.eye(n))) <= 2e-12
+        c.close()
