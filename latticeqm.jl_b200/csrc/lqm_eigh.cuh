@@ -330,6 +330,23 @@ LQM_FN void secular_root_group(bool active, int gw, int g, int k, const double* 
   bool done = !active || k == 1;
   const double dorg = active ? dl[org] : 0.0;
   double tau = (k == 1 && active) ? lo : 0.5 * (lo + hi);
+  if (active && !last) {
+    // first guess (Li's): the two poles around the root as they are, all others at their sum
+    // c in the middle of the interval; with s = |tau| in units of the origin's side
+    const double A = rho * zl[i] * zl[i], Bq = rho * zl[i + 1] * zl[i + 1];
+    const double c = 1.0 + (f0 + (A - Bq) / mid);
+    double x;
+    if (org == i) {  // c x^2 - a x + A gap = 0
+      const double a = c * gap + A + Bq, b = A * gap;
+      const double disc = a * a - 4.0 * b * c, sq = sqrt(disc > 0.0 ? disc : 0.0);
+      x = a > 0.0 ? 2.0 * b / (a + sq) : (a - sq) / (2.0 * c);
+    } else {         // tau = -s: c s^2 - a s - Bq gap = 0
+      const double a = c * gap - A - Bq, b = Bq * gap;
+      const double disc = a * a + 4.0 * b * c, sq = sqrt(disc > 0.0 ? disc : 0.0);
+      x = a < 0.0 ? -2.0 * b / (sq - a) : -(a + sq) / (2.0 * c);
+    }
+    if (x > lo && x < hi) tau = x;
+  }
   for (int it = 0; it < 80; ++it) {
 #if defined(__CUDA_ARCH__)
     if (__all_sync(0xffffffffu, done)) break;
