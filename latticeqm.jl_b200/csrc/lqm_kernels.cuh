@@ -352,16 +352,28 @@ __global__ void __launch_bounds__(256) dos_partial_kernel(const double* __restri
   for (int i0 = 0; i0 < nw; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     const double om = (i < nw) ? omegas[i] : 0.0;
+    // a width, a frequency and values whose squares stay in the normal range (1 / (x^2 + gamma^2)
+    // then does too): quotients without the division's branch, four terms in flight
+    // (500 frequencies, 65536 k-points of n = 24: the call from 9.9 to 9.3 ms)
+    const bool fast = g2 >= 1e-290 && fabs(gamma) < 1e150 && fabs(om) < 1e150;
     double acc = 0.0;
     for (int64_t t0 = b0; t0 < b1; t0 += 1024) {
       const int cnt = (int)((t0 + 1024 < b1) ? 1024 : (b1 - t0));
       __syncthreads();
+      bool wide = false;
       for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
         ev[t] = bands[t0 + t];
         ew[t] = w ? w[(t0 + t) / n] : 1.0;
+        wide = wide || !(fabs(ev[t]) < 1e150) || !(fabs(ew[t]) < 1e150);
       }
-      __syncthreads();
-      if (i < nw) {
+      wide = __syncthreads_or(wide);
+      if (i < nw && fast && !wide) {
+#pragma unroll 4
+        for (int t = 0; t < cnt; ++t) {
+          const double x = om - ev[t];
+          acc += lqm_div_normal(ew[t] * gamma, x * x + g2);
+        }
+      } else if (i < nw) {
         for (int t = 0; t < cnt; ++t) {
           const double x = om - ev[t];
           acc += ew[t] * gamma / (x * x + g2);
