@@ -62,7 +62,8 @@ const char* lqm_last_error(const lqm_ctx* ctx);
  * the earlier copies) or after lqm_ctx_destroy. */
 int lqm_ctx_set_timeout(lqm_ctx* ctx, double seconds);
 /* Eigensolver path selection: orders n >= n_min use the batched blocked path
- * (panel reduction + batched GEMMs); 0 (default) selects it from n = 224 on.
+ * (panel reduction + batched GEMMs); 0 (default) selects it from n = 160 on
+ * (from 224 on where lqm_ctx_set_eigh_threads has set a block size for the order).
  * Below it the staged path (one kernel per stage for a whole list of k-points)
  * serves orders up to 144 and the one-CTA kernel the others; a non-zero n_min
  * holds every order below it to the one-CTA kernel.
@@ -74,10 +75,8 @@ int lqm_ctx_set_blocked_min_n(lqm_ctx* ctx, int64_t n_min);
  * form, one Hermitian mat-vec per column), -1 (default) by order.  Replaces no
  * reference call: the reference's LAPACK zheevr (src/modules/Eigen/Eigen.jl:22-23)
  * reduces in one stage; zheevr_2stage is LAPACK's two-stage form of the same solve.
- * By default the blocked path (n >= 224) takes the two-stage form for passes that
- * return no eigenvectors (bands; rho, which forms only the columns it needs): on
- * B200 1.8x faster for eigenvalue-only passes at n = 1324 and not slower for rho;
- * passes that return all eigenvectors keep the one-stage form. */
+ * By default the blocked path takes the two-stage form, but for passes that return
+ * all eigenvectors above n = 1400, which keep the one-stage form. */
 int lqm_ctx_set_two_stage(lqm_ctx* ctx, int mode);
 /* Device-side wait limit of the bulge chase (the two-stage reduction's stage 2):
  * the polls of a warp's progress word before a wait gives up (0, the default: about

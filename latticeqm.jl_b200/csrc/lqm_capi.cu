@@ -1057,34 +1057,36 @@ bool use_staged(const lqm_ctx* ctx, int n, int nR) {
   return n >= 3 && n <= kStMaxN && nR <= 512 && ctx->blocked_min_n == 0 && !ctx->eigh_nt.count(n);
 }
 
-// Path choice: the blocked path from n = 224 on, or from ctx->blocked_min_n when
-// set, and always beyond the one-CTA kernel's shared-memory plan.  Measured on
-// B200 (disordered honeycomb supercells, 1024 k-points, bands / rho k-points per
-// second, one-CTA kernel against the blocked path): n = 144: 76.6k / 53.1k against
-// 37.1k / 32.9k; n = 196: 31.2k / 19.8k against 23.5k / 18.8k; n = 256: 13.4k /
-// 9.6k against 16.3k / 12.1k; n = 400: 3.2k / 2.3k against 8.2k / 5.0k.
-constexpr int kBlockedDefaultMinN = 224;
+// Path choice: the blocked path from n = 160 on, or from ctx->blocked_min_n when
+// set, and always beyond the one-CTA kernel's shared-memory plan; a block size set for
+// the one-CTA kernel (lqm_ctx_set_eigh_threads) keeps it up to n = 223.  Measured on
+// B200 (honeycomb cells with vacancies, 300 k-points, ms of the eigen pass for bands / rho /
+// all vectors, one-CTA kernel against the blocked path, two-stage): n = 145: 5.4 / 8.5 / 9.0
+// against 3.9 / 7.4 / 7.6, but 1.8 / 2.8 / 3.0 against 2.0 / 3.3 / 3.2 for 8 k-points;
+// n = 176: 8.7 / 14.4 / 13.5 against 5.3 / 8.8 / 9.3 (8 k-points: 2.9 / 4.6 / 4.3 against
+// 1.9 / 3.0 / 2.9); n = 223: 18.9 / 32.2 / 36.1 against 7.7 / 13.5 / 14.4.  160 is also where
+// the blocked path's merges become tiled.
+constexpr int kBlockedDefaultMinN = 160, kOneCtaKeptMaxN = 223;
 bool use_blocked(const lqm_ctx* ctx, int n, int nR) {
-  const int64_t nmin = ctx->blocked_min_n > 0 ? ctx->blocked_min_n : kBlockedDefaultMinN;
+  const int64_t dflt = ctx->eigh_nt.count(n) ? kOneCtaKeptMaxN + 1 : kBlockedDefaultMinN;
+  const int64_t nmin = ctx->blocked_min_n > 0 ? ctx->blocked_min_n : dflt;
   if (n >= nmin) return true;
   return eigh_smem_layout(n, nR, eigh_threads_for(ctx, n), 0).total > 225 * 1024;
 }
 
 // Reduction of the blocked path: two-stage (dense -> band -> tridiagonal) or the
 // one-stage zlatrd panels; ctx->two_stage when set (lqm_ctx_set_two_stage), else the
-// two-stage form from kTwoStageDefaultMinN on (every order the blocked path serves)
-// for passes that return no eigenvectors: eigenvalue-only passes, and density passes,
-// which back-transform only the columns that carry rho_k.  Passes that return all n
-// eigenvectors keep the one-stage reduction: the stage-2 back-transformation of n
-// columns costs 8 n^3 flops per k-point.  Measured on B200 (576 k-points of the
-// 24 x 24 grid unless noted): eigenvalues only at n = 1324 (400-point path) 0.50 s
-// against 0.92 s; rho passes of 1024 k-points: n = 256 70 ms against 78, n = 400 163
-// against 187; n = 508 177 against 178, n = 868 674 against 693, n = 1324 1.90 s
-// against 1.92 s, n = 2884 (144 k-points) 3.94 s against 4.07 s; all vectors (the
-// Hartree-Fock iteration at n = 2884, 144 k-points): 6.5 s against 5.3 s.
+// two-stage form from kTwoStageDefaultMinN on (every order the blocked path serves).
+// Passes that return all n eigenvectors keep the one-stage reduction above
+// kTwoStageVectorsMaxN: the stage-2 back-transformation of n columns costs 8 n^3 flops per
+// k-point.  Measured on B200, ms of the eigen pass with all vectors, one-stage against
+// two-stage: n = 160, 300 k-points 13.4 / 8.0; n = 364, 128 k-points 24.9 / 15.5; n = 676, 100
+// 73 / 60; n = 1000, 64 131 / 109; n = 1324, 64 255 / 224; the gain closes with n and is
+// not measured beyond.  Eigenvalues only at n = 160, 300 k-points: 11.1 / 4.6, rho 14.0 / 7.7.
 // LQM_TWO_STAGE=0/1 in the environment overrides both (development switch for
 // measurements).
 constexpr int kTwoStageDefaultMinN = 128;
+constexpr int kTwoStageVectorsMaxN = 1400;
 bool use_two_stage(const lqm_ctx* ctx, int n, bool all_vectors) {
   if (n <= kTsB + 1) return false;
   const char* env = std::getenv("LQM_TWO_STAGE");
@@ -1092,7 +1094,7 @@ bool use_two_stage(const lqm_ctx* ctx, int n, bool all_vectors) {
   if (ctx->two_stage >= 0) return ctx->two_stage == 1;
   const auto tuned = ctx->two_stage_tuned.find(2 * n + (all_vectors ? 1 : 0));
   if (tuned != ctx->two_stage_tuned.end()) return tuned->second == 1;
-  return !all_vectors && n >= kTwoStageDefaultMinN;
+  return n >= kTwoStageDefaultMinN && (!all_vectors || n <= kTwoStageVectorsMaxN);
 }
 
 int64_t batch_size_for(int64_t n, int64_t nk, double budget_bytes) {

@@ -65,3 +65,28 @@ def test_merges_with_degenerate_levels(lqm, levels):
             assert np.max(np.abs(h[(0, 0)] @ U[:, :, j] - U[:, :, j] * b[:, j])) <= 1e-12
             assert np.max(np.abs(U[:, :, j].conj().T @ U[:, :, j] - np.eye(n))) <= 2e-12
         c.close()
+
+
+@pytest.mark.parametrize("n", [159, 160, 223])
+def test_orders_at_the_default_switch(lqm, n):
+    """The one-CTA kernel, the blocked path, and the one-CTA kernel kept by a set block size."""
+    h = vacancy_cell(n, seed=n)
+    ks = np.random.default_rng(n).uniform(-0.5, 0.5, (2, 3))
+    ref, _ = K.bandmatrix(h, ks)
+    width = np.ptp(ref)
+    rref, eref = K.densitymatrix(h, ks, np.full(3, 1 / 3), 0.1, 0.01, list(h.keys()))
+    for threads in (0, 384):
+        c = lqm.Context()
+        if threads:
+            c.set_eigh_threads(n, threads)
+        b, U = lqm.bandmatrix(h, ks, want_vectors=True, ctx=c)
+        assert np.max(np.abs(b - ref)) <= BAND_TOL * width
+        assert np.max(np.abs(lqm.bandmatrix(h, ks, ctx=c)[0] - ref)) <= BAND_TOL * width
+        for j in range(3):
+            Hk = K.fouriersum(h, ks[:, j])
+            assert np.max(np.abs(Hk @ U[:, :, j] - U[:, :, j] * b[:, j])) <= BAND_TOL * width
+        rho = {R: None for R in h}
+        e = lqm.getdensitymatrix(rho, h, ks, mu=0.1, T=0.01, ctx=c)
+        assert max(np.max(np.abs(rho[R] - rref[R])) for R in h) <= RHO_TOL
+        assert abs(e - eref) <= 1e-9 * max(1.0, n * width)
+        c.close()
