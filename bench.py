@@ -274,7 +274,7 @@ def large_configs(Q, ctx, M, threads):
         "grid": "48x48", "bands_kpts_per_s": ks1.shape[1] / dv, "bands_wall_kpts_per_s": ks1.shape[1] / wl,
         "rho_kpts_per_s": ks1.shape[1] / dd, "rho_wall_kpts_per_s": ks1.shape[1] / wd,
         "cpu_rho_kpts_per_s": cpu_rate(h1, ks1, threads, per_thread=8),
-        "path": "one-CTA-per-k eigensolver, Householder matrix in global scratch (n < 224)"}
+        "path": "staged eigensolver, lower triangle in registers (n <= 144)"}
     # twisted bilayer m=10, n = 1324: the 400-point k-path (bands only; rho on the 24 x 24
     # grid is the headline)
     lat3, h3 = M.tbg_slater_koster(10)

@@ -9,8 +9,11 @@
 //                       partials (summed by the next column step)
 //   blk_finish_kernel   last w of a panel, CTA per k
 //   (host)              rank-2nb trailing update, batched ZGEMM
+//   ts_panel_reg_kernel, ts_w_kernel, ts_band_kernel, ts_chase_kernel, ts_q2g_kernel
+//                       the two-stage reduction and its back-transformation
 //   dc_large_kernel     divide and conquer per k (vectors in global memory,
 //                       tiled merge updates), writes bands and Z (complex)
+//   dc_root_kernel      the last merge's columns of Z, tiles over all k-points
 //   blk_prep_kernel / blk_larft_kernel   compact WY factors per panel
 //   (host)              U = (I - V T V^H) U per panel, batched ZGEMMs
 //   blk_scale_f_kernel  Y = U diag(f), band energy; (host) rho_k = Y U^H
@@ -182,7 +185,6 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc, bool va
 }
 // a hint: the 128-byte line holding *p into L1 (and L2), no register written; callers
 // pass only addresses inside their own buffers
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.L1 [%0];\n" ::"l"(p)); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_keep1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
@@ -685,6 +687,9 @@ __global__ void __launch_bounds__(NT, MINB) dc_large_kernel(DCLargeArgs a) {
 // only for the wanted columns, and with the secular vectors formed as the B tile is
 // staged.  grid (ceil(K / 64), row tiles of both children, nk): 128 x 64 tiles, eight warps of
 // 32 x 32, a ring of three 16-deep stages.  Three quarters of all merge products are this one.
+// Bound by the FP64 tensor path.  With it (and the halved sums below it) the density matrix
+// took 331 ms against 363 at n = 1324 on 144 k-points and 919 against 1232 at n = 2884 on 36,
+// where one block per k-point left three quarters of the SMs idle.
 constexpr int kDcRootThreads = 256;
 constexpr int kDcRootPA = 132, kDcRootPB = 68;  // pitches == 4 mod 16: conflict-free fragment reads
 constexpr int kDcRootStage = 16 * (kDcRootPA + kDcRootPB);
@@ -1063,8 +1068,9 @@ __global__ void __launch_bounds__(kTsPanelThreads, 1) ts_panel_reg_kernel(int n,
 // X = Y T, Z = T^H V^H X.  With G = V^H Y this is W = Y T - V (T^H G T / 2), one pass over V
 // and Y for G and one for W, tensor steps (DMMA) straight from global memory in both; a
 // cluster of cs blocks per k-point, each with a slice of `rows` rows (a multiple of 16).
-// As five to seven GEMM launches this took 84 us per panel at m = 348.  Bound by latency and,
-// for many k-points, by reading V and Y.
+// As five to seven GEMM launches this took 84 us per panel of the n = 364 reduction (32
+// k-points), now 10; 32 us at n = 1324 (144 k-points).  Bound by latency and, for many
+// k-points, by reading V and Y.
 constexpr int kTsWThreads = 256;
 constexpr int kTsWMaxCluster = 8;
 constexpr int kTsWSmem = (kTsWThreads / 32 + kTsWMaxCluster + 4) * kTsB * kTsB * 16;
@@ -1432,7 +1438,10 @@ __global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, doubl
 // as many LSU cycles per step as the arithmetic takes, and all warps at once behind the
 // step's barrier.  So the 16 rows that enter and leave move through a 32-column
 // exchange block per warp, 256 contiguous bytes of a column per half-warp, the entering
-// rows by cp.async one step ahead.
+// rows by cp.async one step ahead.  144 k-points of n = 1324 (693 columns each): 86 ms,
+// 16 TFLOP/s, against 115 ms with direct accesses (256 threads, rows prefetched into L1).
+// Two blocks of 128 let one compute while the other waits at its barrier; 64 and 32 threads,
+// four partial sums, or two reflectors at a time (with their Gram element) are not faster.
 constexpr int kTsQ2gThreads = 128;
 constexpr int kTsQ2gCtas = 2;
 constexpr int kTsQ2gStep = kTsB * kTsB + kTsB;  // complex per staged step
