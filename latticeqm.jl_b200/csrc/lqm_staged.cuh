@@ -18,7 +18,9 @@
 // hetrd, dc, tfac, back, rho; then the one-CTA kernel that ran them before):
 //   n = 24, 16384 k-points: 0.42, 0.85, 0.16, 0.19, 0.10; 9.3
 //   n = 96,  4096 k-points: 3.24, 3.56, 0.19, 0.96, 0.43; 26.8
-//   n = 144, 2304 k-points: 7.45, 6.48, 0.19, 1.87, 0.81; 40.0  The reference's counterpart is LAPACK's zheevr on
+//   n = 144, 2304 k-points: 7.45, 6.48, 0.19, 1.87, 0.81; 40.0
+// (dc before the branch-free quotients and the first guess of the secular roots, which took
+// the whole n = 96 pass on 8100 k-points from 17.5 to 16.3 ms).  The reference's counterpart is LAPACK's zheevr on
 // Hermitian(M) (src/modules/Eigen/Eigen.jl:22-23); the steps are zhetd2, Cuppen's divide and
 // conquer over implicit QL (EISPACK's imtql2), and zlarft / zlarfb.
 #pragma once
