@@ -409,6 +409,11 @@ LQM_FN void secular_root_group(bool active, int gw, int g, int k, const double* 
   *tau_out = tau;
 }
 
+// The order of the values of a merge: ascending, NaN after every number and equal to NaN.  A
+// total order, so that the merged positions and the final places are permutations whatever
+// the values are: the index arrays then have no entry that is read but not written.
+LQM_FN bool dc_less(double a, double b) { return a < b || (b != b && a == a); }
+
 // dlaed2-style deflation for one merge node (single thread), on the values in
 // merged order: zs/ds[lo+p] = z/D of the p-th smallest (gathered in parallel
 // before the scan, so the scan's loads do not wait on each other).
@@ -663,12 +668,12 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
       int cnt = 0;
       if (i < m) {
         int a = m, b = hi;  // first index in [m,hi) with D >= di
-        while (a < b) { int c = (a + b) >> 1; if (S.D[c] < di) a = c + 1; else b = c; }
+        while (a < b) { int c = (a + b) >> 1; if (dc_less(S.D[c], di)) a = c + 1; else b = c; }
         cnt = a - m;
         S.perm[lo + (i - lo) + cnt] = i;
       } else {
         int a = lo, b = m;  // first index in [lo,m) with D > di
-        while (a < b) { int c = (a + b) >> 1; if (S.D[c] <= di) a = c + 1; else b = c; }
+        while (a < b) { int c = (a + b) >> 1; if (!dc_less(di, S.D[c])) a = c + 1; else b = c; }
         cnt = a - lo;
         S.perm[lo + (i - m) + cnt] = i;
       }
@@ -774,8 +779,11 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
       if (nd < 0) continue;
       const int lo = P.lo[nd], hi = P.hi[nd];
       const double v = S.vals[i];
-      int cnt = 0;
-      for (int j = lo; j < hi; ++j) { const double vj = S.vals[j]; cnt += (vj < v) || (vj == v && j < i); }
+      int cnt = 0;  // values before this one by dc_less, equal ones by index
+      if (v == v)
+        for (int j = lo; j < hi; ++j) { const double vj = S.vals[j]; cnt += (vj < v) || (vj == v && j < i); }
+      else
+        for (int j = lo; j < hi; ++j) cnt += S.vals[j] == S.vals[j] || j < i;
       S.newpos[i] = lo + cnt;
     }
     team_sync(T);

@@ -152,6 +152,59 @@ static DCPlan plan_view(const lqm::DCPlanHost& PH) {
   return P;
 }
 
+// Divide and conquer with the last merge left to its record (DCRootRec), as the blocked path
+// runs it.  The index arrays start one past their range, so that an entry that is read before
+// it is written shows.  idx: perm, colnd, newpos, cidx, src (n each) after the solve; returns
+// how many of the last three (and of the poles' limits) are out of range; else Z is formed
+// from the record as dc_root_kernel does.
+extern "C" int lqm_emul_dc_root(int n, const double* d, const double* e, int tile_min, int* idx, double* evals,
+                                double* Z) {
+  const Team T = make_host_team();
+  const lqm::DCPlanHost PH = lqm::make_dc_plan_host(n);
+  const DCPlan PV = plan_view(PH);
+  const size_t nn = (size_t)n * n;
+  std::vector<double> dbuf(13 * (size_t)n + 132), Q(nn + n), Qt(nn + n), Ub(nn), rd(5 * (size_t)n);
+  std::vector<int> ibuf(10 * (size_t)n, n), ri(2 * (size_t)n + 4, n);
+  std::vector<double2> pb((size_t)n + 8);
+  EighVec S;
+  double* db = dbuf.data();
+  S.d = db; S.e = db + n; S.D = db + 2 * n; S.z = db + 3 * n; S.dl = db + 4 * n; S.zl = db + 5 * n;
+  S.troot = db + 6 * n; S.zhat = db + 7 * n; S.vals = db + 8 * n; S.dval = db + 9 * n; S.rc = db + 10 * n;
+  S.rs = db + 11 * n; S.nrho = db + 12 * n; S.red = db + 13 * n;
+  int* ib = ibuf.data();
+  S.perm = ib; S.colnd = ib + n; S.org = ib + 2 * n; S.dcol = ib + 3 * n; S.newpos = ib + 4 * n;
+  S.ri = ib + 5 * n; S.rj = ib + 6 * n; S.nk = ib + 7 * n; S.nrot = ib + 8 * n; S.ndef = ib + 9 * n;
+  S.pbuf = pb.data();
+  DCRootRec R;
+  R.zh = rd.data(); R.dl = R.zh + n; R.lorg = R.dl + n; R.tq = R.lorg + n; R.sc = R.tq + n;
+  R.cidx = ri.data(); R.src = R.cidx + n; R.hdr = R.src + n;
+  std::memcpy(S.d, d, sizeof(double) * n);
+  std::memcpy(S.e, e, sizeof(double) * (n - 1));
+  S.e[n - 1] = 0.0;
+  dc_solve(T, n, PV, S, Q.data(), Qt.data(), nullptr, true, Ub.data(), tile_min, &R);
+  std::memcpy(evals, S.D, sizeof(double) * n);
+  const int k = R.hdr[0], nu = R.hdr[1], nm = R.hdr[2], mid = R.hdr[3];
+  int bad = !(0 <= nu && nu <= nm && nm <= k && k <= n && mid == n / 2);
+  for (int i = 0; i < n; ++i) {
+    idx[i] = S.perm[i]; idx[n + i] = S.colnd[i]; idx[2 * n + i] = S.newpos[i];
+    idx[3 * n + i] = i < k ? R.cidx[i] : 0; idx[4 * n + i] = R.src[i];
+    bad += S.newpos[i] < 0 || S.newpos[i] >= n;
+    bad += idx[3 * n + i] < 0 || idx[3 * n + i] >= n;
+    bad += R.src[i] < -1 || R.src[i] >= n;
+  }
+  if (bad) return bad;
+  for (int c = 0; c < n; ++c)
+    for (int r = 0; r < n; ++r) {
+      double acc = 0.0;
+      if (R.src[c] >= 0) acc = Q[r + (size_t)R.src[c] * n];
+      else
+        for (int p = (r < mid) ? 0 : nu; p < ((r < mid) ? nm : k); ++p)
+          acc += Q[r + (size_t)R.cidx[p] * n] * (R.zh[p] / ((R.dl[p] - R.lorg[c]) - R.tq[c]) * R.sc[c]);
+      Z[r + (size_t)c * n] = acc;
+    }
+  return 0;
+}
+
 // The blocked large-n path on one k-point: panel reduction (blk_column,
 // blk_symv_tile, blk_t12_slab, blk_prev_w; the rank-2nb update done here as loops),
 // divide and conquer with the tiled merge update from tile_min rows on, and
