@@ -602,7 +602,6 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
       }
     bnd[i] = lo;
   }
-  for (int i = tid; i < n; i += NT) S.perm[i] = i;  // in range even where NaN leaves holes in the orders below
   // scale by a power of two to a largest entry in [1/2, 1)
   double mx = 0.0;
   for (int i = tid; i < n; i += NT) {
@@ -640,7 +639,8 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
     ok = st_leaf_ql(s, d, e, Zl, ld, lane) && ok;
     __syncwarp();
     int pos = 0;
-    const long long b = __double_as_longlong(d), key = b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+    const long long b = __double_as_longlong(d);
+    const long long key = d == d ? b ^ ((b >> 63) & 0x7fffffffffffffffLL) : 0x7fffffffffffffffLL;  // NaN last (dc_less)
     for (int j = 0; j < 16; ++j) {
       const long long o = __shfl_sync(FULL, key, (lane & 16) + j);
       pos += j < s && (o < key || (o == key && j < i0));
@@ -748,10 +748,10 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
       const double di = ev[i];
       int p, b, c;
       if (up) {  // first value of the lower half that is >= di
-        for (p = m, b = hi; p < b;) { c = (p + b) >> 1; if (ev[c] < di) p = c + 1; else b = c; }
+        for (p = m, b = hi; p < b;) { c = (p + b) >> 1; if (dc_less(ev[c], di)) p = c + 1; else b = c; }
         p = i + (p - m);
       } else {   // first value of the upper half that is > di
-        for (p = lo, b = m; p < b;) { c = (p + b) >> 1; if (ev[c] <= di) p = c + 1; else b = c; }
+        for (p = lo, b = m; p < b;) { c = (p + b) >> 1; if (!dc_less(di, ev[c])) p = c + 1; else b = c; }
         p = p + (i - m);
       }
       zs[p] = z * 0.70710678118654752440;
@@ -920,8 +920,10 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
       const int q = own[i], lo = nlo[q], hi = nhi[q], it = i - lo, kk = S.nk[q];
       const double v = S.vals[i];
       int pos = lo;
-      for (int j = lo; j < hi; ++j) { const double vj = S.vals[j]; pos += (vj < v) || (vj == v && j < i); }
-      if (!(v == v)) pos = i;
+      if (v == v)
+        for (int j = lo; j < hi; ++j) { const double vj = S.vals[j]; pos += (vj < v) || (vj == v && j < i); }
+      else  // NaN: after every number, by index
+        for (int j = lo; j < hi; ++j) pos += S.vals[j] == S.vals[j] || j < i;
       S.newpos[i] = pos;
       ev[pos] = v;
       // the physical column of this value: a non-deflated value takes that of its place
@@ -1045,7 +1047,9 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
         for (int h = 0; h < 2; ++h) {
           const int it = c0 + 2 * t + h;
           if (it >= i1) continue;
-          double* dst = Zk + (S.newpos[it] - cbeg) * n;
+          const int c = S.newpos[it];
+          if (c < cbeg || c >= cend) continue;  // NaN among the values: the places do not ascend
+          double* dst = Zk + (c - cbeg) * n;
 #pragma unroll
           for (int r = 0; r < RR; ++r) {
             const int row = r < tu ? 8 * r + g : mid + 8 * (r - tu) + g;
