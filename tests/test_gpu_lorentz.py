@@ -46,3 +46,28 @@ def test_conductivity_with_empty_and_full_states(lqm, ctx, T, mu):
     got = lqm.opticalconductivity(om, h, J, J, ks, mu=mu, Gamma=0.05, T=T, ctx=ctx)
     ref = K.opticalconductivity(om, h, J, J, ks, mu=mu, gamma=0.05, T=T)
     assert np.max(np.abs(got - ref)) <= 1e-9 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("gamma", [1e-160, 1e-146, 0.05, 1e149, 1e151])
+@pytest.mark.parametrize("top", [2.0, 1e149, 1e153, 1e170])
+@pytest.mark.parametrize("far", [False, True])
+def test_conductivity_of_distant_levels(lqm, ctx, gamma, top, far):
+    """Uncoupled levels up to 1e170 (squares beyond the largest number: zero terms), widths and
+    frequencies on both sides of the fast form's range: 1e-12 of the terms' magnitudes."""
+    e = np.array([-top, -1.0, 0.3, 1.0, top])
+    n = len(e)
+    rng = np.random.default_rng(0)
+    J = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    J = J + J.conj().T
+    om = np.array([0.0, 0.61, 1e120, 1e151, -1e155][:5 if far else 3])  # one far frequency turns its whole tile
+    got = lqm.opticalconductivity(om, {(0, 0): np.diag(e).astype(complex)}, {(0, 0): J}, {(0, 0): J}, np.zeros((2, 1)),
+                                  mu=0.0, Gamma=gamma, T=0.0, ctx=ctx)
+    f = (e < 0.0).astype(float)
+    off = ~np.eye(n, dtype=bool)
+    wt = ((f[:, None] - f[None, :]) * np.abs(J) ** 2)[off]
+    with np.errstate(over="ignore"):
+        z = (e[:, None] - e[None, :])[off][None] - om[:, None]
+        r = 1.0 / (z * z + gamma * gamma)
+        ref = -1j * (wt * (z + 1j * gamma) * r).sum(1)
+        scale = (np.abs(wt) * (np.abs(z) + gamma) * r).sum(1)
+    assert np.all(np.isfinite(got)) and np.all(np.abs(got - ref) <= 1e-12 * scale)
