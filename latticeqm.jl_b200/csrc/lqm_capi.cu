@@ -1186,8 +1186,13 @@ void chempot_enqueue(lqm_ctx* ctx, int64_t n, int64_t nk, const double* d_bands,
                      double T, double* mu_out, double* err_out) {
   const int64_t nv = n * nk;
   ck(cudaMemsetAsync(err_out, 0, sizeof(double), ctx->stream), "memset");
-  // about four values per thread, one CTA per SM at most
-  const int64_t G = std::max<int64_t>(1, std::min<int64_t>((nv + 4 * kMuThreads - 1) / (4 * kMuThreads), ctx->num_sms));
+  // about four values per thread; one CTA per SM at most, or as many as fit with one step per pass
+  const bool one = T > 0 && nv >= kMuOneStep * ctx->num_sms;
+  const auto kern = one ? mu_search_kernel<1> : mu_search_kernel<kMuLevels>;
+  int per_sm = 1;
+  if (one) ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMuThreads, 0), "occupancy");
+  const int64_t G = std::max<int64_t>(1, std::min<int64_t>((nv + 4 * kMuThreads - 1) / (4 * kMuThreads),
+                                                           (int64_t)std::max(per_sm, 1) * ctx->num_sms));
   double* part = (double*)ws_get(ctx, WS_MU, (size_t)(2 * G * kMuPts) * sizeof(double) + 256);
   MuArgs a;
   a.bands = d_bands; a.n = (int)n; a.nv = nv; a.w = d_w; a.filling = filling; a.T = T;
@@ -1200,7 +1205,7 @@ void chempot_enqueue(lqm_ctx* ctx, int64_t n, int64_t nk, const double* d_bands,
   a.err = err_out;
   ck(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), ctx->stream), "memset");
   void* args[] = {&a};
-  ck(cudaLaunchCooperativeKernel((const void*)mu_search_kernel, dim3((unsigned)G), dim3(kMuThreads), args, 0,
+  ck(cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)G), dim3(kMuThreads), args, 0,
                                  ctx->stream),
      "chemical potential launch");
   ctx->launches += 1;

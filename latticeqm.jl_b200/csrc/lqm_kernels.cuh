@@ -440,6 +440,7 @@ struct MuArgs {
 constexpr int kMuThreads = 256;
 constexpr int kMuLevels = 3;                      // bisection steps per pass over the values
 constexpr int kMuPts = (1 << kMuLevels) - 1;      // points of a pass: every midpoint those steps can ask for
+constexpr int64_t kMuOneStep = 2048;              // T > 0: values per SM from which a pass takes one step
 constexpr int kMuCache = 4096;                    // values a CTA keeps in shared memory
 constexpr int kMuWaitPolls = 1 << 24;             // bound of one grid barrier
 
@@ -451,10 +452,16 @@ constexpr int kMuWaitPolls = 1 << 24;             // bound of one grid barrier
 // launches per step: the values are read once into shared memory.  Bound by the barrier's
 // latency: chemicalpotential() twice (T = 0 and 0.02) at n = 51 on 1024 k-points takes 1.80
 // ms with its eigen passes, 4.87 ms with the 560 and 280 launches of one step each.
+// Three steps by seven points are 7 / 3 evaluations a step.  For T > 0 and long lists that costs
+// more than the barriers it saves, so a pass takes one step (LV = 1) from 2048 values per SM on.
+// Three steps against one, ms of the search on one value in 64: 131 072 values 0.25 / 0.28;
+// 262 144: 0.36 / 0.32; 2 097 152: 2.0 / 0.9; 33.6 million: 35.3 / 14.3 (17.5 with two launches per step).
 //   T > 0: the root of mean f(eps - mu) - filling between the smallest and largest value.
 //   T = 0: the midpoint of two neighbouring order statistics (chemicalpotential.jl:9-23), the
 //          lower one by the same bisection of #{v <= x}, the next one in a last pass.
-__global__ void __launch_bounds__(kMuThreads) mu_search_kernel(MuArgs a) {
+template <int LV>
+__global__ void __launch_bounds__(kMuThreads, LV == 1 ? 3 : 1) mu_search_kernel(MuArgs a) {
+  constexpr int NP = (1 << LV) - 1, MP = NP < 2 ? 2 : NP;  // points of a step's pass, and of any pass
   __shared__ double val[kMuCache];
   __shared__ double red[kMuThreads / 32][kMuPts];
   __shared__ double tot[kMuPts];
@@ -510,20 +517,21 @@ __global__ void __launch_bounds__(kMuThreads) mu_search_kernel(MuArgs a) {
   };
   // tot[p] = mean f(v - x_p) - filling (T > 0) or #{v <= x_p} (T = 0)
   auto evaluate = [&](const double* x, int np) {
-    double s[kMuPts];
+    double s[MP];
 #pragma unroll
-    for (int p = 0; p < kMuPts; ++p) s[p] = 0.0;
+    for (int p = 0; p < MP; ++p) s[p] = 0.0;
+#pragma unroll (LV == 1 ? 4 : 1)
     for (int64_t i = tid; i < cnt; i += kMuThreads) {
       const double v = value(i), wi = a.w ? a.w[(b0 + i) / a.n] : 1.0;
 #pragma unroll
-      for (int p = 0; p < kMuPts; ++p)
+      for (int p = 0; p < MP; ++p)
         if (p < np) {
           if (a.T > 0.0) s[p] = fma(wi, fermi(v - x[p], a.T), s[p]);
           else s[p] += v <= x[p] ? 1.0 : 0.0;  // counts below 2^53: exact
         }
     }
 #pragma unroll
-    for (int p = 0; p < kMuPts; ++p)
+    for (int p = 0; p < MP; ++p)
       if (p < np) {
         s[p] = warp_sum(s[p]);
         if (lane == 0) red[wid][p] = s[p];
@@ -552,7 +560,7 @@ __global__ void __launch_bounds__(kMuThreads) mu_search_kernel(MuArgs a) {
   } else {
     // g(x) > 0 beyond the wanted point; g at the ends first
     const double ends[2] = {lo, hi};
-    double x[kMuPts], fa, fb;
+    double x[MP], fa, fb;
     evaluate(ends, 2);
     const bool warm = a.T > 0.0;
     auto g = [&](double s) { return warm ? s * a.norm - a.filling : s >= (double)a.target ? 1.0 : -1.0; };
@@ -565,28 +573,28 @@ __global__ void __launch_bounds__(kMuThreads) mu_search_kernel(MuArgs a) {
     else if (!warm && fa > 0.0) result = lo;
     else if (sgn(fa) == sgn(fb)) err = 1.0;
     else done = false;
-    for (int it = 0; !done && it < 70 && !lost; ++it) {
+    for (int it = 0; !done && it * LV < 210 && !lost; ++it) {
       // the midpoints of the next steps as a heap: x[q] splits its interval, 2 q + 1 is
       // the split of the lower part, 2 q + 2 of the upper
-      double la[kMuPts], lb[kMuPts];
+      double la[NP], lb[NP];
       la[0] = lo;
       lb[0] = hi;
 #pragma unroll
-      for (int q = 0; q < kMuPts; ++q) {
+      for (int q = 0; q < NP; ++q) {
         x[q] = float_mid(la[q], lb[q]);
-        if (2 * q + 2 < kMuPts) {
+        if (2 * q + 2 < NP) {
           la[2 * q + 1] = la[q]; lb[2 * q + 1] = x[q];
           la[2 * q + 2] = x[q];  lb[2 * q + 2] = lb[q];
         }
       }
-      evaluate(x, kMuPts);
+      evaluate(x, NP);
       int q = 0;
 #pragma unroll
-      for (int s = 0; s < kMuLevels; ++s) {
+      for (int s = 0; s < LV; ++s) {
         if (done) break;
         double m = 0.0, t = 0.0;
 #pragma unroll
-        for (int p = 0; p < kMuPts; ++p)
+        for (int p = 0; p < NP; ++p)
           if (p == q) { m = x[p]; t = tot[p]; }
         if (m == lo || m == hi) {
           result = warm ? (fabs(fa) <= fabs(fb) ? lo : hi) : hi;
