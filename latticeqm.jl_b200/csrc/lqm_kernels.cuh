@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(kMuThreads, LV == 1 ? 3 : 1) mu_search_kernel(
     const bool warm = a.T > 0.0;
     auto g = [&](double s) { return warm ? s * a.norm - a.filling : s >= (double)a.target ? 1.0 : -1.0; };
     fa = g(tot[0]);
-    fb = g(tot[1]);
+    fb = warm ? g(tot[1]) : 1.0;  // T = 0: the largest value where NaN keeps the count below the target
     __syncthreads();
     bool done = true;
     if (warm && fa == 0.0) result = lo;
