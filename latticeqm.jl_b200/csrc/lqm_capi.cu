@@ -1074,6 +1074,13 @@ bool use_blocked(const lqm_ctx* ctx, int n, int nR) {
   return eigh_smem_layout(n, nR, eigh_threads_for(ctx, n), 0).total > 225 * 1024;
 }
 
+// Orders that the one-CTA kernel takes where it is asked for (the several-models launch): those
+// below lqm_ctx_set_blocked_min_n or, by default, up to kOneCtaKeptMaxN.
+bool one_cta_serves(const lqm_ctx* ctx, int n, int nR) {
+  const int64_t nmin = ctx->blocked_min_n > 0 ? ctx->blocked_min_n : kOneCtaKeptMaxN + 1;
+  return n < nmin && eigh_smem_layout(n, nR, eigh_threads_for(ctx, n), 0).total <= 225 * 1024;
+}
+
 // Reduction of the blocked path: two-stage (dense -> band -> tridiagonal) or the
 // one-stage zlatrd panels; ctx->two_stage when set (lqm_ctx_set_two_stage), else the
 // two-stage form from kTwoStageDefaultMinN on (every order the blocked path serves).
@@ -1296,7 +1303,7 @@ void launch_eigh_multi(lqm_ctx* ctx, int nm, const lqm_hops* const* H, int64_t n
   int NT = 0;
   for (int m = 0; m < nm; ++m) {
     const int n = (int)H[m]->n;
-    if (use_blocked(ctx, n, (int)H[m]->nR))
+    if (!one_cta_serves(ctx, n, (int)H[m]->nR))
       fail(LQM_EINVAL, "model %d (n=%d) is served by the blocked eigensolver, not the one-CTA one", m, n);
     tnt[m] = eigh_threads_for(ctx, n);
     NT = std::max(NT, tnt[m]);
