@@ -476,7 +476,7 @@ def batch_config(Q, ctx, M, torch, dev, np, steps, fp64_peak):
         detail[f"n{s_['n']}"] = {"eigh_ms_per_step": ms / steps, "eigh_tflops": tf,
                                  "eigh_frac_of_fp64": (tf / fp64_peak) if tf else None,
                                  "eigh_block_size": block_sizes.get(f"n{s_['n']}")}
-    # the same step with ONE eigensolver launch for the three models (sub-teams per CTA)
+    # the same step as one call for the three models
     multi = [dict(H=s_["Hd"], Lk=s_["Lk"], rho=s_["rho"], om=s_["om"], dos=s_["dos"], bands=s_["bands"])
              for s_ in state]
     for _ in range(3):
@@ -489,17 +489,18 @@ def batch_config(Q, ctx, M, torch, dev, np, steps, fp64_peak):
     e1.record()
     torch.cuda.synchronize()
     el1 = e0.elapsed_time(e1) / 1e3
-    eigh_ms1, eigh_launches1, _ = ctx.stats()
+    eigh_ms1, eigh_passes1, launches1 = ctx.stats()
     for s_ in state:
         s_["Hd"].free()
     return {"workload": BATCH_WORKLOAD, "kpts_per_s": len(state) * nk * steps / el, "ms_per_step": 1000 * el / steps,
             "steps": steps, "warmup": 3, "per_model": detail,
             "eigh_flops_per_k": "8 nR n^2 + 13.33 n^3 (Bloch sum + eigh with vectors; rho_k fused, not counted)",
             "one_launch": {"kpts_per_s": len(state) * nk * steps / el1, "ms_per_step": 1000 * el1 / steps,
-                           "eigh_launches_per_step": eigh_launches1 / steps, "eigh_ms_per_step": eigh_ms1 / steps,
-                           "note": "lqm_bands_dos_rho_multi_dev: the three models' k-points in one eigensolver "
-                                   "launch (CTA sub-teams of each model's block size), then the per-model folds "
-                                   "and DOS"}}
+                           "eigh_passes_per_step": eigh_passes1 / steps,
+                           "kernel_launches_per_step": launches1 / steps, "eigh_ms_per_step": eigh_ms1 / steps,
+                           "note": "lqm_bands_dos_rho_multi_dev: one call for the three models (staged eigen passes "
+                                   "model after model, or one launch of CTA sub-teams where a block size is set), "
+                                   "then the per-model folds and DOS"}}
 
 
 def main():

@@ -136,12 +136,14 @@ int lqm_autotune_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double*
 /* Milliseconds of device time of the last call's kernels (CUDA events). */
 int lqm_ctx_last_kernel_ms(const lqm_ctx* ctx, double* ms);
 
-/* Device-time statistics since the last reset: eigh_ms / eigh_launches cover
- * the per-k eigensolver kernel, launches counts every kernel this library
- * launched.  The reset also sets what is recorded: enable_timing 0 = nothing,
- * 1 = CUDA-event timing of the eigensolver launches, 2 = that plus the
- * per-phase SM cycle counters of lqm_ctx_phase_cycles (clock reads inside the
- * kernel, so a profiling mode, not a timing one). */
+/* Device-time statistics since the last reset: eigh_ms is the device time of the eigen
+ * passes and eigh_launches their number (one per k-list or chunk of it, whatever the
+ * number of kernels of its path; one for all models of a several-models call); launches
+ * counts every kernel this library launched (a replayed graph's once, when captured).
+ * The reset also sets what is recorded: enable_timing 0 = nothing, 1 = CUDA-event timing
+ * of the eigen passes, 2 = that plus the per-phase SM cycle counters of
+ * lqm_ctx_phase_cycles (clock reads inside the kernels, so a profiling mode, not a
+ * timing one). */
 int lqm_ctx_reset_stats(lqm_ctx* ctx, int enable_timing);
 int lqm_ctx_stats(const lqm_ctx* ctx, double* eigh_ms, int64_t* eigh_launches, int64_t* launches);
 /* The same statistics per kernel class: 0 = the eigensolver passes (as above),

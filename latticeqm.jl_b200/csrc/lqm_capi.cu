@@ -427,6 +427,7 @@ void zgemm_sb(lqm_ctx* ctx, GemmOp ta, GemmOp tb, int m, int n, int k, double al
     const int64_t mn = (int64_t)m * n;
     zgemm_split_reduce_kernel<<<(unsigned)std::min<int64_t>((mn + 255) / 256, 8 * ctx->num_sms), 256, 0, h>>>(
         m, n, nsplit, P, beta_re, C, ldc, 0, 1);
+    ctx->launches++;  // the sum (the callers count the product)
     ck(cudaGetLastError(), "zgemm split launch");
     return;
   }
@@ -445,6 +446,7 @@ void zgemm_sb(lqm_ctx* ctx, GemmOp ta, GemmOp tb, int m, int n, int k, double al
       const int64_t tot = (int64_t)m * n * batch;
       zgemm_split_reduce_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 8 * ctx->num_sms), 256, 0, h>>>(
           m, n, ns, P, beta_re, C, ldc, sC, batch);
+      ctx->launches++;
       ck(cudaGetLastError(), "zgemm split launch");
       return;
     }
@@ -966,7 +968,7 @@ void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const doubl
       else if (n <= 96) launch_st_back<12, 2>(ctx, ba);
       else if (n <= 128) launch_st_back<16, 1>(ctx, ba);
       else launch_st_back<18, 1>(ctx, ba);
-      ctx->launches += 3;
+      ctx->launches += 2;
       if (part) {
         const int64_t nt = (n + 31) / 32;
         const StRhoArgs oa{n, nb, U, nullptr, occ, ncol, comp, rk.rhok, phases};
@@ -1121,6 +1123,7 @@ void launch_fold(lqm_ctx* ctx, int64_t nn, int64_t nb, const double2* rk, const 
   NvtxRange nvtx_("rho fold");
   zgemm_sb(blas_handle(ctx), OP_N, OP_T, (int)nn, nL, (int)nb, 1.0, rk, (int)nn, 0, coef, nL, 0,
            accumulate ? 1.0 : 0.0, d_rho, (int)nn, 0, 1);
+  ctx->launches++;
 }
 
 // bands_out (n x nk, device) receives every k's eigenvalues when non-null.

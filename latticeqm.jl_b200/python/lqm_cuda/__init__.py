@@ -203,13 +203,13 @@ class Context:
         return v.value
 
     def reset_stats(self, timing=True, phases=False):
-        """Zero the statistics; ``timing`` records CUDA-event times of the eigensolver
-        launches, ``phases`` also its per-phase cycle counters (see ``phase_cycles``)."""
+        """Zero the statistics; ``timing`` records CUDA-event times of the eigen
+        passes, ``phases`` also their per-phase cycle counters (see ``phase_cycles``)."""
         mode = 2 if phases else int(bool(timing))
         self.check(_lib.lqm_ctx_reset_stats(self._h, mode))
 
     def stats(self):
-        """(eigensolver device ms, eigensolver launches, all kernel launches) since reset."""
+        """(device ms of the eigen passes, number of eigen passes, kernel launches) since reset."""
         ms, el, al = _D(), _I64(), _I64()
         self.check(_lib.lqm_ctx_stats(self._h, ctypes.byref(ms), ctypes.byref(el), ctypes.byref(al)))
         return ms.value, el.value, al.value
@@ -1101,7 +1101,7 @@ def scf_hf_gradient(h, v, rho, mu, ks, T=0.0, kweights=None, eps_bar=None, beta=
 
 def bands_dos_rho_multi_dev(models, d_ks, nk, mu=0.0, T=0.01, gamma=0.05, d_w=None, ctx=None):
     """``lqm_bands_dos_rho_multi_dev``: bands, DOS and rho_L of several models on one k list
-    (device arrays) with ONE eigensolver launch.  ``models``: list of dicts with
+    (device arrays) with one eigen pass over all of them.  ``models``: list of dicts with
     ``H`` (DeviceHops), ``Lk`` (keys d x nL int64, F order), ``rho`` (device nL x n x n
     complex), ``om`` (device omegas), ``dos`` (device nw), ``bands`` (device nk x n).
     Returns the band energies."""
