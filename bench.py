@@ -442,8 +442,8 @@ def batch_config(Q, ctx, M, torch, dev, np, steps, fp64_peak):
     block_sizes = {}
     for s_ in state:
         if s_["n"] < 128:
-            best, _, table = Q.autotune_eigh(s_["Hd"], ks_np, want_rho=True, ctx=ctx)
-            block_sizes[f"n{s_['n']}"] = best
+            Q.autotune_eigh(s_["Hd"], ks_np, want_rho=True, ctx=ctx)
+            block_sizes[f"n{s_['n']}"] = ctx.eigh_threads(s_["n"]) or "built-in rule (staged path)"
     eb = ctypes.c_double()
 
     def step(per_model_ms=None):

@@ -115,22 +115,27 @@ int lqm_ctx_scf_exchange_energy(const lqm_ctx* ctx, double* eJ);
  * rule, under which orders up to 144 take the staged path instead.  No reference
  * counterpart (a device launch parameter). */
 int lqm_ctx_set_eigh_threads(lqm_ctx* ctx, int64_t n, int nt);
+/* The context's choice for order n, as lqm_ctx_set_eigh_threads takes it: the block size
+ * that was set or autotuned, 0 where the built-in rule stands.  Given to another context
+ * it makes that one run the same kernels. */
+int lqm_ctx_get_eigh_threads(const lqm_ctx* ctx, int64_t n, int* nt);
 /* Autotuner of that block size for H's order (below the blocked path): every
  * candidate (the block sizes 32, 64, 128, 256, 384 and 512 from half the
  * built-in rule's size up to four times it, or 512, whose shared-memory plan
  * fits) runs the eigen pass on the nk sample k-points (rho_k at mu = 0, T = 0.01
  * when want_rho, else eigenvectors), warmed up once and timed once with CUDA
- * events; the fastest becomes the context's block size for n, and n keeps the staged
- * path where that is faster than all of them (the sample should
- * span several waves of CTAs, e.g. the production k-grid, or it times latency
- * rather than throughput).  best_nt/best_ms
- * receive the choice, cand_nt/cand_ms (up to ncand_max, may be NULL) every
- * candidate, *ncand their number.  Block sizes differ in rounding, so a choice is
+ * events; the fastest becomes the context's block size for n, unless the built-in rule
+ * has another path for n (the staged one) that is faster than all of them: then n stays
+ * with the rule (the sample should span several waves of CTAs, e.g. the production
+ * k-grid, or it times latency rather than throughput).  best_nt/best_ms receive the
+ * fastest block size and its time, cand_nt/cand_ms (up to ncand_max, may be NULL) every
+ * block size, *ncand their number; the choice itself, to be saved, is what
+ * lqm_ctx_get_eigh_threads then gives.  Choices differ in rounding, so one is
  * meant to be made once and reused.  For an order on the blocked path the
  * reduction is tuned instead: candidates 0 (one-stage) and 1 (two-stage), timed the
  * same way for the sample's pass kind (rho_k when want_rho, else all eigenvectors);
  * the faster is kept for that order and kind unless lqm_ctx_set_two_stage fixed the
- * reduction (then LQM_EINVAL).  No reference counterpart. */
+ * reduction (then block sizes up to n = 223, and LQM_EINVAL beyond).  No reference counterpart. */
 int lqm_autotune_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* ks, int want_rho, int* best_nt,
                       double* best_ms, int64_t ncand_max, int* cand_nt, double* cand_ms, int64_t* ncand);
 /* Milliseconds of device time of the last call's kernels (CUDA events). */

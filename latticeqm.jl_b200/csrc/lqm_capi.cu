@@ -59,8 +59,7 @@ struct lqm_ctx {
   int num_sms = 0;
   double last_ms = 0.0;
   std::map<int, PlanDev> plans;
-  std::map<int, int> eigh_nt;     // one-CTA eigensolver block size per order n where that kernel was chosen (set or autotuned)
-  std::map<int, int> eigh_nt_alt; // autotuned block size where the staged path was faster (the kernel's other uses)
+  std::map<int, int> eigh_nt;  // one-CTA eigensolver block size per order n where that kernel was chosen (set or autotuned)
   DevBuf ws[64];
   // per-kernel device-time statistics (CUDA events on the context stream)
   bool stats_on = false;
@@ -321,11 +320,8 @@ int eigh_threads(int n) { return n <= 16 ? 32 : (n <= 32 ? 64 : (n < 64 ? 128 : 
 // The block size of the one-CTA eigensolver for order n on this context: the value
 // set by lqm_ctx_set_eigh_threads / lqm_autotune_eigh, else the rule above.
 int eigh_threads_for(const lqm_ctx* ctx, int n) {
-  for (const auto* m : {&ctx->eigh_nt, &ctx->eigh_nt_alt}) {
-    const auto it = m->find(n);
-    if (it != m->end()) return it->second;
-  }
-  return eigh_threads(n);
+  const auto it = ctx->eigh_nt.find(n);
+  return it != ctx->eigh_nt.end() ? it->second : eigh_threads(n);
 }
 
 // eigh_kernel instantiation for a block size.  Blocks of up to 128 threads
@@ -1493,9 +1489,15 @@ int lqm_ctx_scf_exchange_energy(const lqm_ctx* ctx, double* eJ) {
   return LQM_OK;
 }
 
+int lqm_ctx_get_eigh_threads(const lqm_ctx* ctx, int64_t n, int* nt) {
+  if (!ctx || n < 1 || !nt) return LQM_EINVAL;
+  const auto it = ctx->eigh_nt.find((int)n);
+  *nt = it != ctx->eigh_nt.end() ? it->second : 0;
+  return LQM_OK;
+}
+
 int lqm_ctx_set_eigh_threads(lqm_ctx* ctx, int64_t n, int nt) {
   if (!ctx || n < 1 || nt < 0 || nt > 512 || nt % 32 != 0) return LQM_EINVAL;
-  ctx->eigh_nt_alt.erase((int)n);
   if (nt == 0) ctx->eigh_nt.erase((int)n);
   else ctx->eigh_nt[(int)n] = nt;
   return LQM_OK;

@@ -306,7 +306,8 @@ function cuda_wilson_wannier2d(H, NX::Int, NY::Int, bands::AbstractVector{<:Inte
 end
 
 """Autotune the one-CTA eigensolver's block size for H's order on sample k-points
-(`lqm_autotune_eigh`); the choice stays on the device's context.  Returns
+(`lqm_autotune_eigh`); the choice stays on the device's context (an order that is faster
+on another path stays there) and is `cuda_get_eigh_threads(n, exec)`.  Returns
 (best block size, its ms, Dict(block size => ms))."""
 function cuda_autotune_eigh(H, ks::AbstractMatrix{Float64}, exec::CudaExec; want_rho::Bool=true)
     ctx = context(exec.device)
@@ -325,6 +326,15 @@ end
 cuda_set_two_stage(mode::Int, exec::CudaExec) =
     check(context(exec.device), ccall((:lqm_ctx_set_two_stage, LIB[]), Cint, (Ptr{Cvoid}, Cint),
                                       context(exec.device).ptr, mode))
+
+"""The choice for order n as `cuda_set_eigh_threads` takes it: a block size, or 0 for the
+built-in rule."""
+function cuda_get_eigh_threads(n::Int, exec::CudaExec)
+    ctx = context(exec.device)
+    nt = Ref{Cint}(0)
+    check(ctx, ccall((:lqm_ctx_get_eigh_threads, LIB[]), Cint, (Ptr{Cvoid}, Int64, Ref{Cint}), ctx.ptr, n, nt))
+    Int(nt[])
+end
 
 """Set the one-CTA eigensolver's block size for order n (0: the built-in rule)."""
 cuda_set_eigh_threads(n::Int, nt::Int, exec::CudaExec) =

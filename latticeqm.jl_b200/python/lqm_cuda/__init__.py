@@ -47,7 +47,7 @@ EXPORTS = [
     "lqm_commutator_norm", "lqm_ctx_set_scf_residual", "lqm_ctx_set_scf_terms", "lqm_ctx_set_scf_exchange",
     "lqm_ctx_scf_exchange_energy", "lqm_hartreefock_eval", "lqm_bdg_densitymatrix", "lqm_bdg_filling",
     "lqm_bdg_chemicalpotential", "lqm_scf_hf_bdg", "lqm_berry_flux", "lqm_berry_path", "lqm_fermisurface",
-    "lqm_wilson", "lqm_wilson_wannier", "lqm_ctx_set_eigh_threads", "lqm_autotune_eigh", "lqm_ctx_kernel_stats",
+    "lqm_wilson", "lqm_wilson_wannier", "lqm_ctx_set_eigh_threads", "lqm_ctx_get_eigh_threads", "lqm_autotune_eigh", "lqm_ctx_kernel_stats",
     "lqm_comm_unique_id", "lqm_ctx_set_comm", "lqm_ctx_comm", "lqm_shard_range", "lqm_scf_hf_gradient",
     "lqm_bands_dos_rho_multi_dev",
 ]
@@ -115,6 +115,7 @@ _SIG = {
     "lqm_wilson": [_P, _P, _I64, _I64, _I64, _P, ctypes.c_int, _P, _P],
     "lqm_wilson_wannier": [_P, _P, _I64, _I64, _I64, _P, _P, _P],
     "lqm_ctx_set_eigh_threads": [_P, _I64, ctypes.c_int],
+    "lqm_ctx_get_eigh_threads": [_P, _I64, ctypes.POINTER(ctypes.c_int)],
     "lqm_autotune_eigh": [_P, _P, _I64, _P, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(_D), _I64,
                           _P, _P, ctypes.POINTER(_I64)],
     "lqm_fermisurface": [_P, _P, _I64, _P, _I64, _P, _D, _P, _P, ctypes.POINTER(_D)],
@@ -196,6 +197,13 @@ class Context:
     def set_eigh_threads(self, n, nt):
         """Block size of the one-CTA eigensolver for order n (0: the built-in rule)."""
         self.check(_lib.lqm_ctx_set_eigh_threads(self._h, int(n), int(nt)))
+
+    def eigh_threads(self, n):
+        """The choice for order n as set_eigh_threads takes it: a block size, or 0 for the
+        built-in rule (``lqm_ctx_get_eigh_threads``)."""
+        nt = ctypes.c_int()
+        self.check(_lib.lqm_ctx_get_eigh_threads(self._h, int(n), ctypes.byref(nt)))
+        return nt.value
 
     def last_kernel_ms(self):
         v = _D()
@@ -762,7 +770,9 @@ def wilson_wannier2d(H, NX, NY=0, bands=(0,), ctx=None):
 def autotune_eigh(H, ks, want_rho=True, ctx=None):
     """Times every candidate block size of the one-CTA eigensolver for H's order on the
     sample k-points ``ks`` (the rho_k pass when ``want_rho``, else eigenvectors) and keeps
-    the fastest on the context (``lqm_autotune_eigh``): (best_nt, best_ms, {nt: ms}).
+    the fastest on the context (``lqm_autotune_eigh``): (best_nt, best_ms, {nt: ms}); an
+    order that is faster on another path (the staged one) stays there.  The choice to be
+    saved for ``Context.set_eigh_threads`` is ``Context.eigh_threads(n)``.
     For an order on the blocked path the candidates are the reductions instead, 0
     (one-stage) and 1 (two-stage), kept for that order and pass kind."""
     ctx = ctx or default_context()
