@@ -380,6 +380,24 @@ void launch_zgemm_dmma(cudaStream_t st, const GemmArgs& g, int batch) {
   zgemm_dmma_kernel<BM, BN, WM, WN, BK, ST><<<grid, nt, smem, st>>>(g);
 }
 
+// Raises fn's limit of dynamic shared memory to bytes.  The limit belongs to the process, not to
+// a context, so it is never lowered: with the size of an order as the limit, a host thread
+// working on a smaller order could set its own between another's call here and its launch,
+// which is then refused.
+template <class F>
+cudaError_t raise_smem(F* fn, size_t bytes) {
+  static std::mutex m;
+  const std::lock_guard<std::mutex> lock(m);
+  cudaFuncAttributes at{};
+  const cudaError_t e = cudaFuncGetAttributes(&at, fn);
+  if (e != cudaSuccess || (size_t)at.maxDynamicSharedSizeBytes >= bytes) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+template <class F>
+void set_smem(F* fn, size_t bytes) {
+  ck(raise_smem(fn, bytes), "smem attr");
+}
+
 // kernel<<<cs nk, nt, smem>>>(args...) in clusters of cs blocks
 template <class... P, class... Q>
 void launch_cluster(cudaStream_t st, void (*kernel)(P...), int cs, int64_t nk, int nt, int smem, Q... args) {
@@ -612,9 +630,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
     ck(cudaMalloc(&ctx->d_err, sizeof(int)), "cudaMalloc(error word)");
     ck(cudaMemset(ctx->d_err, 0, sizeof(int)), "memset(error word)");
   }
-  ck(cudaFuncSetAttribute(dc_large_kernel<kDcThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          dc_tile_smem(n)),
-     "smem attr");
+  set_smem(dc_large_kernel<kDcThreads, 1>, dc_tile_smem(n));
   std::pair<cudaEvent_t, cudaEvent_t> evs{};
   if (ctx->stats_on) { evs = stat_events(ctx); ck(cudaEventRecord(evs.first, ctx->stream), "event"); }
   for (int64_t k0 = 0; k0 < nk; k0 += B) {
@@ -785,7 +801,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
         ctx->launches++;
       }
       const size_t lsm = (size_t)g2 * sizeof(double2);
-      ck(cudaFuncSetAttribute(blk_larft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm), "smem attr");
+      set_smem(blk_larft_kernel, lsm);
       blk_larft_kernel<<<dim3((unsigned)P2, (unsigned)nbk), kBlkThreads, lsm, ctx->stream>>>(n, nbt, P2, A, tau,
                                                                                              Tm, G, off);
       ctx->launches++;
@@ -846,11 +862,6 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
 }
 
 // ---- staged path (lqm_staged.cuh) ----
-template <class F>
-void set_smem(F* fn, size_t bytes) {
-  ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attr");
-}
-
 template <int WR, int WC, int NB, int KEPT, int MINB>
 void launch_st_hetrd(lqm_ctx* ctx, const StHetrdArgs& a) {
   const size_t sm = st_hetrd_complex<StGrid<WR, WC, NB, KEPT>>(a.nR) * sizeof(double2);
@@ -993,7 +1004,7 @@ void launch_eigh_one(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* 
   if (!a_in_smem) Ls = eigh_smem_layout(n, (int)H->nR, nt, 0);
   if (Ls.total > 225 * 1024) fail(LQM_EINVAL, "n=%d, nR=%lld exceeds the shared-memory plan", n, (long long)H->nR);
   const EighFn kfn = eigh_fn(nt);
-  ck(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ls.total), "smem attr");
+  set_smem(kfn, Ls.total);
   int per_sm = 0;
   ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, nt, Ls.total), "occupancy");
   if (per_sm < 1) fail(LQM_EINVAL, "eigh kernel cannot be resident for n=%d", n);
@@ -1342,7 +1353,7 @@ void launch_eigh_multi(lqm_ctx* ctx, int nm, const lqm_hops* const* H, int64_t n
   }
   ma.slots_per_cta = slots_per_cta;
   auto kfn = NT == 384 ? &eigh_multi_kernel<384> : &eigh_multi_kernel<512>;
-  ck(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+  set_smem(kfn, (size_t)smem);
   int per_sm = 0;
   ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, NT, (size_t)smem), "occupancy");
   if (per_sm < 1) fail(LQM_EINVAL, "the model-batched eigensolver cannot be resident");
@@ -2133,8 +2144,7 @@ extern "C" int lqm_bandmatrix_noalloc(void* stream, int64_t n, int64_t nR, int32
   const int64_t max_slots = kNoAllocScratchDoubles / slot;
   if (max_slots < 1) return LQM_EINVAL;  // one k-point's scratch exceeds the 64 MiB array
   const EighFn kfn = eigh_fn(nt);
-  if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ls.total) != cudaSuccess)
-    return LQM_ECUDA;
+  if (raise_smem(kfn, Ls.total) != cudaSuccess) return LQM_ECUDA;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, nt, Ls.total) != cudaSuccess ||
       per_sm < 1)
