@@ -522,6 +522,169 @@ extern "C" int lqm_emul_chase_schedules(int n, int b, const double* band, int wo
   return -1;
 }
 
+// The same chase by the device kernel's pairs (ts_chase_kernel): pair p takes the sweeps p,
+// p + pairs, ...; its maker forms a task's reflector and updates the block below, its applier
+// does the rest of the task behind it.  The pair's state is the kernel's: three blocks that
+// rotate by the pair's count of tasks, two reflectors with their scalars, one meeting per
+// task, the applier's progress word, the maker's halt flag.  Pauses vary the interleaving;
+// a plain read or write that the protocol does not order is a data race here too.  Returns 1
+// where band, reflectors and taus equal the sequential chase's bit for bit, 0 where they
+// differ, 2 where a wait of more than `limit` polls made every pair stop (0: no limit).
+template <int B>
+static int emul_chase_pairs(int n, const double* band, int pairs, unsigned seed, long long limit) {
+  const Team T = make_host_team();
+  constexpr int LW = B + 1;
+  const int ldb = 2 * B, tmax = ts_tmax(n, B);
+  const size_t nb = (size_t)ldb * n, nv = (size_t)std::max(n - 1, 1) * tmax;
+  std::vector<double2> B1(nb), B2(nb), V1(nv * B), V2(nv * B), t1(nv), t2(nv);
+  std::memcpy(B1.data(), band, nb * sizeof(double2));
+  std::memcpy(B2.data(), band, nb * sizeof(double2));
+  std::vector<double2> win(3 * B * LW + 2 * B);
+  for (int s = 0; s <= n - 2; ++s)
+    ts_chase_sweep<B>(T, n, s, B1.data(), V1.data() + (size_t)s * tmax * B, t1.data() + (size_t)s * tmax, win.data(),
+                      [](int) { return true; }, [](int) {});
+  struct Pair {
+    double2 blk[3][B * LW], v[2][B], tau[2], beta[2];
+    std::atomic<int> arrived{0}, turn{0};
+    int halt = 0;
+    void meet() {
+      const int mine = turn.load(std::memory_order_acquire);
+      if (arrived.fetch_add(1, std::memory_order_acq_rel) == 1) {
+        arrived.store(0, std::memory_order_relaxed);
+        turn.store(mine + 1, std::memory_order_release);
+      } else {
+        while (turn.load(std::memory_order_acquire) == mine) std::this_thread::yield();
+      }
+    }
+  };
+  std::vector<Pair> P(pairs);
+  std::vector<std::atomic<long long>> prog(pairs);
+  for (auto& p : prog) p.store(-1);
+  std::atomic<int> stop{0};
+  const long long unit = tmax + 1;
+  double2* Bd = B2.data();
+  auto rest = [](std::mt19937& rng) {
+    if (rng() % 16 == 0) std::this_thread::sleep_for(std::chrono::microseconds(rng() % 50));
+  };
+  auto maker = [&](int w) {
+    std::mt19937 rng(seed * 7919u + (unsigned)w);
+    Pair& q = P[w];
+    const int wp = (w + pairs - 1) % pairs;
+    int it = 0;
+    for (int s = w; s <= n - 2; s += pairs) {
+      const int nt = ts_tasks(n, B, s), ntp = s > 0 ? ts_tasks(n, B, s - 1) : 0;
+      for (int t = 0; t < nt; ++t, ++it) {
+        const int R0 = s + 1 + t * B, R1 = R0 + B, L = std::min(B, n - R0), L2 = std::min(B, std::max(n - R1, 0));
+        bool ok = true;
+        if (s > 0) {
+          const long long need = (long long)(s - 1) * unit + std::min(t + 3, ntp);
+          for (long long polls = 0; ok && prog[wp].load(std::memory_order_acquire) < need; std::this_thread::yield()) {
+            if (stop.load()) ok = false;
+            else if (limit > 0 && ++polls > limit) { stop.store(1); ok = false; }
+          }
+        }
+        if (!ok) {
+          q.halt = 1;
+          q.meet();
+          return;
+        }
+        double2* X = q.blk[it % 3];
+        double2* EN = q.blk[(it + 1) % 3];
+        double2* v = q.v[it & 1];
+        if (t == 0)
+          for (int r = 0; r < L; ++r) X[r] = ts_bget(Bd, ldb, R0 + r, s);
+        for (int c = 0; c < L; ++c)
+          for (int r = 0; r < L2; ++r) EN[r + c * LW] = ts_bget(Bd, ldb, R1 + r, R0 + c);
+        double s2 = 0.0, beta;
+        for (int r = 1; r < L; ++r) s2 += X[r].x * X[r].x + X[r].y * X[r].y;
+        double2 tj, scal;
+        zlarfg_scalars(X[0], s2, &tj, &beta, &scal);
+        const size_t slot = (size_t)s * tmax + t;
+        for (int r = 0; r < B; ++r)
+          V2[slot * B + r] = v[r] = r == 0 ? cmk(1.0, 0.0) : r < L ? cmul(scal, X[r]) : cmk(0.0, 0.0);
+        t2[slot] = q.tau[it & 1] = tj;
+        q.beta[it & 1] = cmk(beta, 0.0);
+        for (int i = 0; i < L2; ++i) {
+          double2 acc = cmk(0.0, 0.0);
+          for (int c = 0; c < L; ++c) acc = cadd(acc, cmul(EN[i + c * LW], v[c]));
+          const double2 z = cmul(tj, acc);
+          for (int c = 0; c < L; ++c) EN[i + c * LW] = csub(EN[i + c * LW], cmul(z, cconj(v[c])));
+        }
+        rest(rng);
+        q.meet();
+      }
+    }
+  };
+  auto applier = [&](int w) {
+    std::mt19937 rng(seed * 104729u + (unsigned)w);
+    Pair& q = P[w];
+    std::vector<double2> D(B * LW), y(B);
+    int it = 0;
+    for (int s = w; s <= n - 2; s += pairs) {
+      const int nt = ts_tasks(n, B, s);
+      for (int t = 0; t < nt; ++t, ++it) {
+        q.meet();
+        if (q.halt) return;
+        rest(rng);
+        const int R0 = s + 1 + t * B, c = t == 0 ? s : R0 - B, L = std::min(B, n - R0);
+        double2* X = q.blk[it % 3];
+        const double2* v = q.v[it & 1];
+        const double2 tj = q.tau[it & 1];
+        for (int k = 0; k < L; ++k)
+          for (int r = k; r < L; ++r) D[r + k * LW] = ts_bget(Bd, ldb, R0 + r, R0 + k);
+        for (int r = 0; r < L; ++r) X[r] = r == 0 ? q.beta[it & 1] : cmk(0.0, 0.0);
+        if (t > 0)
+          for (int l = 1; l < B; ++l) {
+            double2* f = X + l * LW;
+            double2 acc = cmk(0.0, 0.0);
+            for (int r = 0; r < L; ++r) acc = cadd(acc, cmulc(v[r], f[r]));
+            const double2 fl = cmul(cconj(tj), acc);
+            for (int r = 0; r < L; ++r) f[r] = csub(f[r], cmul(v[r], fl));
+          }
+        for (int l = 0; l < (t > 0 ? B : 1); ++l)
+          for (int r = 0; r < L; ++r) *ts_bptr(Bd, ldb, R0 + r, c + l) = X[r + l * LW];
+        double g = 0.0;
+        for (int r = 0; r < L; ++r) {
+          double2 acc = cmk(0.0, 0.0);
+          for (int k = 0; k < L; ++k) acc = cadd(acc, cmul(k <= r ? D[r + k * LW] : cconj(D[k + r * LW]), v[k]));
+          g += cmulc(v[r], acc).x;
+          y[r] = acc;
+        }
+        const double h = -0.5 * (tj.x * tj.x + tj.y * tj.y) * g;
+        for (int r = 0; r < L; ++r) y[r] = cadd(cmul(tj, y[r]), cscale(h, v[r]));
+        for (int r = 0; r < L; ++r)
+          for (int k = 0; k <= r; ++k) {
+            double2 a = csub(D[r + k * LW], cadd(cmul(y[r], cconj(v[k])), cmul(v[r], cconj(y[k]))));
+            if (k == r) a.y = 0.0;
+            *ts_bptr(Bd, ldb, R0 + r, R0 + k) = a;
+          }
+        prog[w].store((long long)s * unit + t + 1, std::memory_order_release);
+      }
+    }
+  };
+  std::vector<std::thread> th;
+  for (int w = 0; w < pairs; ++w) {
+    th.emplace_back(maker, w);
+    th.emplace_back(applier, w);
+  }
+  for (auto& t : th) t.join();
+  if (stop.load()) return 2;
+  bool same = std::memcmp(B1.data(), B2.data(), nb * sizeof(double2)) == 0;
+  for (int s = 0; s <= n - 2 && same; ++s)
+    for (int t = 0; t < ts_tasks(n, B, s) && same; ++t) {
+      const size_t q = (size_t)s * tmax + t;
+      same = std::memcmp(&V1[q * B], &V2[q * B], B * sizeof(double2)) == 0 &&
+             std::memcmp(&t1[q], &t2[q], sizeof(double2)) == 0;
+    }
+  return same ? 1 : 0;
+}
+
+extern "C" int lqm_emul_chase_pairs(int n, int b, const double* band, int pairs, unsigned seed, long long limit) {
+  if (b == 4) return emul_chase_pairs<4>(n, band, pairs, seed, limit);
+  if (b == 16) return emul_chase_pairs<16>(n, band, pairs, seed, limit);
+  return -1;
+}
+
 // rho_from_U on a given U (n x n, ld n) and occupations f.
 extern "C" int lqm_emul_rho(int n, const double* U, const double* f, double* out) {
   const Team T = make_host_team();
