@@ -85,6 +85,11 @@ int lqm_ctx_set_two_stage(lqm_ctx* ctx, int mode);
  * the context then serves later calls.  A small limit makes the waits run out on
  * purpose (a test of that path; no fault is involved).  No reference counterpart. */
 int lqm_ctx_set_device_wait_limit(lqm_ctx* ctx, int64_t polls);
+/* QL sweeps that the staged path (orders up to 144) gives a leaf of its divide and conquer
+ * (0, the default: 480, about fifteen times what is needed).  A k-point with a leaf that is
+ * not done by then is solved again by the one-CTA kernel; a small limit sends k-points there
+ * on purpose (a test of that route).  No reference counterpart. */
+int lqm_ctx_set_leaf_sweeps(lqm_ctx* ctx, int sweeps);
 /* SCF acceleration of lqm_scf_hf on this context: 0 (default) linear damped
  * mixing, 1..8 Anderson (Type-II) acceleration with that history depth
  * (src/modules/Meanfield/fixedpoint.jl:39-194,201-231: acceleration=:anderson,

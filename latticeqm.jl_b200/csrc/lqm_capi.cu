@@ -101,6 +101,7 @@ struct lqm_ctx {
   // wait_stream reads it once such a kernel has been launched since the last check
   int* d_err = nullptr;
   bool err_armed = false;
+  int leaf_sweeps = 0;  // QL sweeps of a leaf of the staged path (0: the default)
   int64_t dev_wait_limit = 0;  // polls before a device-side wait of the bulge chase gives up (0: the default)
   // NCCL communicator of the k-point shards (lqm_ctx_set_comm; lqm_comm.inc)
   void* comm = nullptr;
@@ -959,7 +960,7 @@ void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const doubl
     if (ro) rk = RhoOut{ro->rhok + k0 * nn, ro->ebk + k0, ro->w + k0, ro->mu, ro->T};
     const bool part = ro && !d_U;  // only the columns that carry rho_k
     const StDcArgs da{n, st_depth(n), nb, d, e, bands, Z, rk.mu, rk.T, rk.w, part ? rk.ebk : nullptr, occ, ncol, comp,
-                      redo, phases};
+                      redo, ctx->leaf_sweeps > 0 ? ctx->leaf_sweeps : kStLeafSweeps, phases};
     if (n <= 32) launch_st_dc<32, 1, 4, 16>(ctx, da);
     else if (n <= 64) launch_st_dc<128, 4, 8, 4>(ctx, da);
     else if (n <= 96) launch_st_dc<256, 6, 12, 2>(ctx, da);
@@ -986,7 +987,7 @@ void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const doubl
       }
       ck(cudaGetLastError(), "staged back-transformation launch");
     }
-    // k-points of which a leaf did not converge (none in practice)
+    // k-points of which a leaf did not converge (none in practice; NaN, or lqm_ctx_set_leaf_sweeps)
     launch_eigh_one(ctx, H, nb, d_ks + k0 * H->d, bands, d_U ? U : nullptr, ro ? &rk : nullptr, redo);
   }
   if (ctx->stats_on) { ck(cudaEventRecord(evs.second, ctx->stream), "event"); ctx->ev_pending.push_back(evs); }
@@ -1523,6 +1524,12 @@ int lqm_ctx_set_blocked_min_n(lqm_ctx* ctx, int64_t n_min) {
 int lqm_ctx_set_device_wait_limit(lqm_ctx* ctx, int64_t polls) {
   if (!ctx || polls < 0) return LQM_EINVAL;
   ctx->dev_wait_limit = polls;
+  return LQM_OK;
+}
+
+int lqm_ctx_set_leaf_sweeps(lqm_ctx* ctx, int sweeps) {
+  if (!ctx || sweeps < 0) return LQM_EINVAL;
+  ctx->leaf_sweeps = sweeps;
   return LQM_OK;
 }
 

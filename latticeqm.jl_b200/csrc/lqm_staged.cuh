@@ -428,6 +428,7 @@ struct StDcArgs {
   int* ncol;        // nk: packed columns
   int* comp;        // nk: 1 where rho_k = I + sum of the (negative) weights
   int* redo;        // nk flags: 1 where a leaf did not converge; then their count (zeroed before)
+  int sweeps;       // QL sweeps of a leaf at most
   unsigned long long* phase_cycles;
 };
 
@@ -450,16 +451,16 @@ __host__ __device__ inline size_t st_dc_doubles(int n, bool vec) {
 // count comes from a vote or is a constant, so that the warp stays together and only
 // assignments are conditional.  An off-diagonal entry is dropped below eps (|d_i| +
 // |d_{i+1}|) + eps / 16 (of a matrix scaled to a largest entry below one).  Returns false
-// where kStLeafSweeps sweeps were not enough (about 2 s are needed).
+// where `sweeps` were not enough (about 2 s are needed).
 constexpr int kStLeafSweeps = 30 * kStLeaf;
-__device__ __forceinline__ bool st_leaf_ql(int s, double& d, double& e, double* Zl, int ld, int lane) {
+__device__ __forceinline__ bool st_leaf_ql(int s, double& d, double& e, double* Zl, int ld, int lane, int sweeps) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr double EPS = 2.0 * LQM_DEPS;
   const int i0 = lane & 15, half = lane & 16;
   const bool row = i0 < s;
   int l = 0;
   unsigned rem = 1;
-  for (int sweep = 0; sweep < kStLeafSweeps; ++sweep) {
+  for (int sweep = 0; sweep < sweeps; ++sweep) {
     const double dn = __shfl_down_sync(FULL, d, 1);
     const bool tiny = i0 >= s - 1 || fabs(e) <= EPS * (fabs(d) + fabs(dn)) + EPS / 16.0;
     const unsigned mask = (__ballot_sync(FULL, tiny) >> half) & 0xffffu;  // bit i: no coupling of i and i + 1
@@ -636,7 +637,7 @@ __global__ void __launch_bounds__(NT, MINB) st_dc_kernel(StDcArgs a) {
     if (i0 < s)
       for (int c = 0; c < s; ++c) Zl[i0 + c * ld] = i0 == c ? 1.0 : 0.0;
     __syncwarp();
-    ok = st_leaf_ql(s, d, e, Zl, ld, lane) && ok;
+    ok = st_leaf_ql(s, d, e, Zl, ld, lane, a.sweeps) && ok;
     __syncwarp();
     int pos = 0;
     const long long b = __double_as_longlong(d);
