@@ -368,8 +368,8 @@ def measured_fp64_peak(torch, dev):
 
 
 def profile_case(Q, ctx, h, torch, dev, np):
-    """A small case of the bench's dominant kernel for profilers: 2048 k-points of the
-    n=96 model through lqm_bands_dos_rho_dev (one eigh_kernel launch)."""
+    """A small case of the staged eigensolver for profilers: 2048 k-points of the n=96 model
+    through lqm_bands_dos_rho_dev, twice."""
     nk = 2048
     ks = np.random.default_rng(0).random((2, nk))
     d_ks = torch.from_numpy(np.ascontiguousarray(ks.T)).to(dev)
@@ -422,7 +422,7 @@ def profile_case_kubo(Q, ctx, M):
 def batch_config(Q, ctx, M, torch, dev, np, steps, fp64_peak):
     """The batched three-model configuration (n = 8, 24, 96; 256 x 256 k each): bands +
     DOS + rho_R through lqm_bands_dos_rho_dev with device-resident inputs, 3 warm-up
-    steps and `steps` timed steps; the one-CTA eigensolver's FP64 roofline per model."""
+    steps and `steps` timed steps; the eigen pass's FP64 roofline per model."""
     models = M.batch_models()
     ks_np = kgrid(0, 1)
     nk = ks_np.shape[1]

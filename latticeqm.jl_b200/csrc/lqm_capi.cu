@@ -277,7 +277,7 @@ enum WsSlot {
   WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_VU, WS_VB, WS_VX, WS_VT, WS_VG, WS_ONES, WS_SCFY, WS_AND, WS_EXCH, WS_HFPART, WS_BDG, WS_BDGE, WS_BDGI, WS_BDGK, WS_BDGP, WS_BDGB, WS_CSC, WS_UNIW, WS_SPAN, WS_GRAD, WS_GRADE, WS_HFPART2, WS_GEMMSPLIT, WS_GRAM, WS_TSP, WS_TSB, WS_TSV2,
   WS_STV, WS_STZ, WS_STU, WS_STI, WS_STOCC, WS_LDCQ, WS_LDCREC
 };
-static_assert(WS_STOCC < 64, "workspace slots");
+static_assert(WS_LDCREC < 64, "workspace slots");  // the last of the list
 
 }  // namespace
 #include "lqm_comm.inc"
@@ -1074,8 +1074,9 @@ bool use_staged(const lqm_ctx* ctx, int n, int nR) {
 // all vectors, one-CTA kernel against the blocked path, two-stage): n = 145: 5.4 / 8.5 / 9.0
 // against 3.9 / 7.4 / 7.6, but 1.8 / 2.8 / 3.0 against 2.0 / 3.3 / 3.2 for 8 k-points;
 // n = 176: 8.7 / 14.4 / 13.5 against 5.3 / 8.8 / 9.3 (8 k-points: 2.9 / 4.6 / 4.3 against
-// 1.9 / 3.0 / 2.9); n = 223: 18.9 / 32.2 / 36.1 against 7.7 / 13.5 / 14.4.  160 is also where
-// the blocked path's merges become tiled.
+// 1.9 / 3.0 / 2.9); n = 223: 18.9 / 32.2 / 36.1 against 7.7 / 13.5 / 14.4.  The rule looks at
+// n alone: the orders below 160, where the longer list and the shorter one want different
+// kernels, stay where they were.  160 is also where the blocked path's merges become tiled.
 constexpr int kBlockedDefaultMinN = 160, kOneCtaKeptMaxN = 223;
 bool use_blocked(const lqm_ctx* ctx, int n, int nR) {
   const int64_t dflt = ctx->eigh_nt.count(n) ? kOneCtaKeptMaxN + 1 : kBlockedDefaultMinN;
@@ -1098,8 +1099,10 @@ bool one_cta_serves(const lqm_ctx* ctx, int n, int nR) {
 // kTwoStageVectorsMaxN: the stage-2 back-transformation of n columns costs 8 n^3 flops per
 // k-point.  Measured on B200, ms of the eigen pass with all vectors, one-stage against
 // two-stage: n = 160, 300 k-points 13.4 / 8.0; n = 364, 128 k-points 24.9 / 15.5; n = 676, 100
-// 73 / 60; n = 1000, 64 131 / 109; n = 1324, 64 255 / 224; the gain closes with n and is
-// not measured beyond.  Eigenvalues only at n = 160, 300 k-points: 11.1 / 4.6, rho 14.0 / 7.7.
+// 73 / 60; n = 1000, 64 131 / 109; n = 1324, 64 255 / 224; n = 1588, 64 386 / 365;
+// n = 1876, 64 596 / 567; n = 2884, 36 1210 / 1174.  Beyond 1400 the few per cent that it gains
+// are left for its memory: the stage-2 reflectors take a further n^2 complex per k-point, so
+// that a batch holds fewer.  Eigenvalues only at n = 160, 300 k-points: 11.1 / 4.6, rho 14.0 / 7.7.
 // LQM_TWO_STAGE=0/1 in the environment overrides both (development switch for
 // measurements).
 constexpr int kTwoStageDefaultMinN = 128;

@@ -183,8 +183,6 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc, bool va
   const int nbytes = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled, nothing is read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(nbytes) : "memory");
 }
-// a hint: the 128-byte line holding *p into L1 (and L2), no register written; callers
-// pass only addresses inside their own buffers
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_keep1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 

@@ -28,7 +28,7 @@
 
 namespace lqm {
 
-constexpr int kStMaxN = 144;    // the lower triangle in the registers of eight warps
+constexpr int kStMaxN = 144;    // the lower triangle in four warps' registers and, above 64, shared memory
 constexpr int kStNB = 8;        // reflectors per compact-WY block
 
 __host__ __device__ inline int st_chunks(int n) { return (n + 31) / 32; }

@@ -1,5 +1,7 @@
 // Two-stage Hermitian tridiagonalisation for the batched large-n path, written
-// as team phases so the CUDA kernels and the host emulation share the arithmetic.
+// as team phases: the defining forms.  The band extraction and, beyond 4096 rows, the panel QR
+// run on the device as they stand here; the panel in registers, the chase and the grouped
+// back-transformation have kernels of their own (lqm_large.cuh).
 //
 //   stage 1, dense -> band of half-bandwidth b (LAPACK zhetrd_he2hb, lower): per
 //     panel of b columns a QR of the m x b block below the band (ts_panel_qr),
@@ -181,8 +183,9 @@ LQM_FN void ts_band_extract(const TeamT& T, int n, const double2* A, int lda, do
 // task's), and F, x and D go back to the band once they are final.  wait(t) is
 // called before task t's loads (false: give up, the sweep returns false) and done(t)
 // after its stores.  vout / tauout (or null): task t's v (B complex, zero-padded)
-// at vout + t B and tau at tauout[t].  The defining form, against which the emulation
-// checks the device's pipeline of the same tasks (ts_chase_kernel).
+// at vout + t B and tau at tauout[t].  The defining form: the device runs the
+// same tasks on pairs of warps (ts_chase_kernel), and the emulation checks that protocol, on
+// pairs of host threads with its own scalar blocks, against this one bit for bit.
 template <int B, class TeamT, class WaitF, class DoneF>
 LQM_FN bool ts_chase_sweep(const TeamT& T, int n, int s, double2* Bd, double2* vout, double2* tauout,
                            double2* win, WaitF wait, DoneF done) {

@@ -187,8 +187,8 @@ class Context:
 
     def set_two_stage(self, mode):
         """Reduction of the blocked eigensolver: 1 two-stage (dense -> band -> tridiagonal),
-        0 one-stage panels, -1 (default): two-stage on the blocked path for passes that
-        return no eigenvectors."""
+        0 one-stage panels, -1 (default): two-stage, but for passes that return all
+        eigenvectors above n = 1400."""
         self.check(_lib.lqm_ctx_set_two_stage(self._h, int(mode)))
 
     def set_device_wait_limit(self, polls):
