@@ -175,8 +175,8 @@ __device__ __forceinline__ void st_pass(double2 (&A)[G::NA][G::NB], double2* sA,
 //   w = tau' q - 1/2 |tau'|^2 gamma x,   next column = a - x conj(w_o) - w conj(x_o).
 // Per step: the pass, a barrier, then warp 1 takes beta and tau while warp 0 sums t and
 // x^H t, and warp 0 the rest; a barrier.  Bound by instruction issue and the latency of a
-// step's serial part (n = 96: 1.7 instructions per cycle and SM with three CTAs, a third of
-// them FP64; the FP64 pipe is 20% busy).  With the triangle in shared memory it took 6.37 ms
+// step's serial part (n = 96: 1.55 instructions per cycle and SM with three CTAs, a third of
+// them FP64; the FP64 pipe is 27% busy).  With the triangle in shared memory it took 6.37 ms
 // at n = 96 and 4096 k-points, with eight warps per k-point 3.95, without the blocks in
 // shared memory (two CTAs per SM) 3.93.
 template <class G>
