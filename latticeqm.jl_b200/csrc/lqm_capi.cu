@@ -101,6 +101,7 @@ struct lqm_ctx {
   // wait_stream reads it once such a kernel has been launched since the last check
   int* d_err = nullptr;
   bool err_armed = false;
+  double batch_share = 1.0;  // of the eigen passes' batch budgets: halved where the device's memory ran out
   int leaf_sweeps = 0;  // QL sweeps of a leaf of the staged path (0: the default)
   int64_t dev_wait_limit = 0;  // polls before a device-side wait of the bulge chase gives up (0: the default)
   // NCCL communicator of the k-point shards (lqm_ctx_set_comm; lqm_comm.inc)
@@ -585,7 +586,7 @@ void launch_eigh_large(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double
   const int root_mid = n / 2;
   const double per_k = 16.0 * (double)nn * ((vec && !d_U) ? 2.0 : 1.0) + (root ? 8.0 * (double)nn : 0.0) + 16.0 * (double)(auxk + tspk + tsbk + tsvk) +
                        16.0 * n;
-  int64_t B = std::max<int64_t>(1, std::min<int64_t>(nk, (int64_t)(64.0e9 / per_k)));
+  int64_t B = std::max<int64_t>(1, std::min<int64_t>(nk, (int64_t)(64.0e9 * ctx->batch_share / per_k)));
   B = std::min<int64_t>(B, 65535);
   {  // batches of equal size (no short tail batch)
     const int64_t nbat = (nk + B - 1) / B;
@@ -910,7 +911,7 @@ void launch_st_rho_from_U(lqm_ctx* ctx, int n, int64_t nk, const double2* U, con
   ctx->launches += 2;
 }
 
-// Batches of about 4 GB of work buffers.
+// Batches of about 4 GB of work buffers (less where memory is short, see fitting_batches).
 void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands,
                         double2* d_U, const RhoOut* ro) {
   NvtxRange nvtx_("eigen pass (staged)");
@@ -919,7 +920,7 @@ void launch_eigh_staged(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const doubl
   const bool vec = d_U || ro;
   const int P = st_panels(n);
   const double per_k = 16.0 * nn + 32.0 * n + (vec ? 24.0 * nn + 1024.0 * P + 8.0 * n : 0.0);
-  const int64_t B = std::min<int64_t>(nk, std::max<int64_t>(32, (int64_t)(4.0e9 / per_k)));
+  const int64_t B = std::min<int64_t>(nk, std::max<int64_t>(32, (int64_t)(4.0e9 * ctx->batch_share / per_k)));
   double2* V = (double2*)ws_get(ctx, WS_STV, (size_t)B * (nn + 2 * n) * sizeof(double2));
   double2* tau = V + B * nn;
   double* d = (double*)(tau + B * n);
@@ -1032,6 +1033,30 @@ void launch_eigh_one(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* 
   ctx->launches++;
 }
 
+// Runs an eigen pass of the staged or the blocked path.  Where its work buffers (up to 4 and
+// 64 GB, against the few hundred MB of the one-CTA kernel, which served orders up to 223
+// before) do not fit beside what else is on the device, they are given back and the pass runs
+// again in batches of half the size, which the context then keeps.
+template <class F>
+void fitting_batches(lqm_ctx* ctx, F&& pass) {
+  for (;;) {
+    try {
+      pass();
+      return;
+    } catch (const LqmError& e) {
+      if (e.code != LQM_ENOMEM || ctx->batch_share < 1.0 / 512) throw;
+    }
+    cudaGetLastError();  // the failed allocation
+    wait_stream(ctx);
+    for (int s : {WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_LDCQ, WS_LDCREC, WS_TSP, WS_TSB, WS_TSV2, WS_GRAM, WS_STV, WS_STZ,
+                  WS_STU, WS_STI}) {
+      cudaFree(ctx->ws[s].p);
+      ctx->ws[s] = DevBuf{};
+    }
+    ctx->batch_share *= 0.5;
+  }
+}
+
 // Eigen pass over nk device k-points: bands (n x nk), optionally U and/or rho_k.
 bool use_staged(const lqm_ctx* ctx, int n, int nR);
 void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks, double* d_bands, double2* d_U,
@@ -1039,12 +1064,14 @@ void launch_eigh(lqm_ctx* ctx, const lqm_hops* H, int64_t nk, const double* d_ks
   NvtxRange nvtx_("eigen pass");
   const int n = (int)H->n;
   if (use_blocked(ctx, n, (int)H->nR)) {
-    launch_eigh_large(ctx, H, nk, d_ks, d_bands, d_U, ro ? ro->rhok : nullptr, ro ? ro->ebk : nullptr,
-                      ro ? ro->w : nullptr, ro ? ro->mu : 0.0, ro ? ro->T : 0.0);
+    fitting_batches(ctx, [&] {
+      launch_eigh_large(ctx, H, nk, d_ks, d_bands, d_U, ro ? ro->rhok : nullptr, ro ? ro->ebk : nullptr,
+                        ro ? ro->w : nullptr, ro ? ro->mu : 0.0, ro ? ro->T : 0.0);
+    });
     return;
   }
   if (use_staged(ctx, n, (int)H->nR)) {
-    launch_eigh_staged(ctx, H, nk, d_ks, d_bands, d_U, ro);
+    fitting_batches(ctx, [&] { launch_eigh_staged(ctx, H, nk, d_ks, d_bands, d_U, ro); });
     ctx->eigh_launches++;
     return;
   }
@@ -1308,7 +1335,7 @@ void launch_eigh_multi(lqm_ctx* ctx, int nm, const lqm_hops* const* H, int64_t n
   if (staged) {
     for (int m = 0; m < nm; ++m) {
       const RhoOut ro{rhok[m], ebk[m], d_w, mu, T};
-      launch_eigh_staged(ctx, H[m], nk, d_ks, bands[m], nullptr, &ro);
+      fitting_batches(ctx, [&] { launch_eigh_staged(ctx, H[m], nk, d_ks, bands[m], nullptr, &ro); });
     }
     ctx->eigh_launches++;  // one pass over all models
     return;
