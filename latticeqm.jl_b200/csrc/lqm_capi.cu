@@ -132,6 +132,7 @@ namespace {
 
 void ck(cudaError_t e, const char* what) {
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here; else the thread's next launch check reports it once more
     if (e == cudaErrorMemoryAllocation) fail(LQM_ENOMEM, "%s: %s", what, cudaGetErrorString(e));
     fail(LQM_ECUDA, "%s: %s", what, cudaGetErrorString(e));
   }
@@ -1046,7 +1047,6 @@ void fitting_batches(lqm_ctx* ctx, F&& pass) {
     } catch (const LqmError& e) {
       if (e.code != LQM_ENOMEM || ctx->batch_share < 1.0 / 512) throw;
     }
-    cudaGetLastError();  // the failed allocation
     wait_stream(ctx);
     for (int s : {WS_LA, WS_LU, WS_LAUX, WS_LDC, WS_LDCQ, WS_LDCREC, WS_TSP, WS_TSB, WS_TSV2, WS_GRAM, WS_STV, WS_STZ,
                   WS_STU, WS_STI}) {

@@ -50,3 +50,29 @@ def test_passes_fit_the_memory_that_is_left(lqm, n, nk, vectors):
     else:
         assert np.max(np.abs(b - b0)) <= 1e-12 * width
         assert np.max(np.abs(b[:, ::1000] - ref)) <= 1e-10 * width
+
+
+def test_a_refused_call_is_not_reported_again(lqm):
+    """Eigenvectors of 2.4 GB with 0.5 GB left are refused; the next call, on the same and on
+    another context, is served."""
+    import torch
+    h = vacancy_cell(96)
+    c = lqm.Context(0, timeout=600)
+    small = L.regulargrid(4)
+    want = lqm.bandmatrix(h, small, ctx=c)[0]
+    held = []
+    try:
+        torch.cuda.empty_cache()
+        while torch.cuda.mem_get_info()[0] > 2**29 + 2**28:
+            held.append(torch.empty(int(min(torch.cuda.mem_get_info()[0] - 2**29, 2**33)), dtype=torch.uint8,
+                                    device="cuda"))
+        with pytest.raises(lqm.LQMError, match="ENOMEM"):
+            lqm.bandmatrix(h, L.regulargrid(128 * 128), want_vectors=True, ctx=c)
+        assert np.array_equal(lqm.bandmatrix(h, small, ctx=c)[0], want)
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    other = lqm.Context(0, timeout=600)
+    assert np.array_equal(lqm.bandmatrix(h, small, ctx=other)[0], want)
+    other.close()
+    c.close()
