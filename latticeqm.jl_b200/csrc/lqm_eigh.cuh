@@ -607,7 +607,10 @@ struct DCRootRec {
 // Ub (n*n doubles, or null) enables the tiled update for heights whose largest
 // merge has >= tile_min rows: node [lo, hi) keeps its normalised secular
 // vectors at Ub + lo*n as the rows of a k x k block (vector it at it + p*k).
-template <class TeamT>
+// TILED false leaves that form out of the code (the one-CTA kernel, which never takes it):
+// beside it the columns' sums were compiled to a third more time there (n = 158, 1024
+// k-points: 2.39 G cycles of its CTAs against 1.69; the pass with vectors 26.0 ms against 24.6).
+template <bool TILED = true, class TeamT>
 LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S, double* Q, double* Qt,
                               unsigned long long* sub = nullptr, bool vec = true, double* Ub = nullptr,
                               int tile_min = 1 << 30, const DCRootRec* root = nullptr) {
@@ -827,10 +830,10 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
       }
     }
     bool tiled = false;
-    if (vec && Ub != nullptr)
+    if (TILED && vec && Ub != nullptr)
       for (int nd = h0; nd < h1; ++nd) tiled = tiled || (P.hi[nd] - P.lo[nd] >= tile_min);
-    const bool defer = tiled && root != nullptr && h == P.nheights - 1;  // one node, the whole matrix
-    if (tiled) {
+    const bool defer = TILED && tiled && root != nullptr && h == P.nheights - 1;  // one node, the whole matrix
+    if (TILED && tiled) {
       // the child that each column comes from (1 upper, 2 lower, 3 both after a rotation) in
       // S.z, then the order of the poles by it in S.perm and its limits in S.nrot, S.ndef
       for (int i = T.tid; i < n; i += T.nt)
@@ -889,7 +892,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
         }
       }
       if (T.tid == 0) { root->hdr[0] = k; root->hdr[1] = S.nrot[h0]; root->hdr[2] = S.ndef[h0]; root->hdr[3] = P.mid[h0]; }
-    } else if (tiled) {
+    } else if (TILED && tiled) {
       // the secular vectors into Ub, row p of the k x k block by lanes over the columns
       for (int nd = h0; nd < h1; ++nd) {
         const int lo = P.lo[nd], k = S.nk[nd];
@@ -959,7 +962,7 @@ LQM_FN_NOINLINE void dc_solve(const TeamT& T, int n, const DCPlan& P, EighVec& S
         for (int r = lo + T.lane; r < hi; r += T.nl) dst[r] = src[r];
       }
     };
-    for (int t = T.wid; 2 * t < n && vec && !tiled; t += T.nw) {
+    for (int t = T.wid; 2 * t < n && vec && !(TILED && tiled); t += T.nw) {
       const int ca = 2 * t, cb = 2 * t + 1;
       const int nda = own[ca], ndb = (cb < n) ? own[cb] : -1;
       bool pair = false;

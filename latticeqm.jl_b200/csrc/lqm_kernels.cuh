@@ -142,7 +142,7 @@ __device__ __forceinline__ void eigh_point(const TeamT& T, const EighArgs& a, in
     team_sync(T);
   }
   P.tick(PH_HETRD);
-  dc_solve(T, n, a.plan, S, Q, Qt, P.on ? P.dsub : nullptr, need_vec);
+  dc_solve<false>(T, n, a.plan, S, Q, Qt, P.on ? P.dsub : nullptr, need_vec);
   for (int i = T.tid; i < n; i += T.nt) a.bands[k * n + i] = S.D[i];
   P.tick(PH_DC);
   if (need_vec) {
