@@ -485,14 +485,17 @@ void zgemm_sb(lqm_ctx* ctx, GemmOp ta, GemmOp tb, int m, int n, int k, double al
     launch_zgemm_dmma<64, 64, 16, 32, 8, 3>(h, g, batch);
   else {
     // the tile that computes least: for orders that are no multiple of 64 the padding of
-    // 64 x 64 tiles is most of the work (n = 72: 128 x 128).  The smaller tiles load more
-    // per product, counted as a tenth and a twentieth.  Measured, all four products of the
+    // 64 x 64 tiles is most of the work (n = 72: 128 x 128).  Per element computed, padding
+    // included, 72 x 24 tiles reach 20.5 TFLOP/s in large batches where 64 x 64 and 48 x 48 reach
+    // 30: counted as 1.46, and 1.05 for 48 x 48 and its further loads.  n = 200, 264 and 400, 16
+    // matrices, 72 x 24 / 64 x 64 / 48 x 48: 11.4 / 14.2 / 15.7, 14.3 / 13.6 / 18.1 and 17.3 /
+    // 21.6 / 24.6.  Measured, all four products of the
     // density VJP at n = 72 on 1296 k-points: 0.93 ms against 1.76 on 64 x 64 tiles; the two
     // of the conductivity at n = 144 on 2304: 3.72 against 6.51 on 48 x 48 tiles.
     auto cost = [&](int bm, int bn, double f) {
       return f * ((m + bm - 1) / bm * (double)bm) * ((n + bn - 1) / bn * (double)bn);
     };
-    const double c64 = cost(64, 64, 1.0), c72 = cost(72, 24, 1.1), c48 = cost(48, 48, 1.05);
+    const double c64 = cost(64, 64, 1.0), c72 = cost(72, 24, 1.46), c48 = cost(48, 48, 1.05);
     if (c64 <= c72 && c64 <= c48) launch_zgemm_dmma<64, 64, 32, 32, 8, 3>(h, g, batch);
     else if (c72 <= c48) launch_zgemm_dmma<72, 24, 24, 24, 8, 3>(h, g, batch);
     else launch_zgemm_dmma<48, 48, 24, 24, 8, 3>(h, g, batch);
