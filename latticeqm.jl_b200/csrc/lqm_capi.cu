@@ -475,10 +475,19 @@ void zgemm_sb(lqm_ctx* ctx, GemmOp ta, GemmOp tb, int m, int n, int k, double al
   // 64 x 16 tiles against 16.3 / 11.5 on 128 x 16; U -= V Y (k = 64, n = 693) at m = 1200 /
   // 300: 23.9 / 22.1 on 32 x 32 against 23.3 / 20.7 on 64 x 64 of eight warps.  V^H U
   // (m = 64) has a long k and keeps 64 x 64, its warps 16 x 32: 28.4 against 24.8 for 32 x 32.
-  if (n <= 16)
+  // One tall product (the fold of rho_R, m = n^2) is bound by reading A and writing C, and from
+  // about 32768 rows on wants the larger tiles while k is short: m = 160000, k = 16 / 64 / 144,
+  // n = 9: 128 x 16 against 64 x 16 1.37, 1.16, 1.06 times as fast; n = 64, k = 16 / 64: 64 x 64
+  // against 32 x 32 1.56, 1.15 (even at k = 400, and at 22500 rows; slower below).
+  const bool tall = batch == 1 && m >= 32768;
+  if (n <= 16 && tall && k < 256)
+    launch_zgemm_dmma<128, 16, 16, 16, 8, 3>(h, g, batch);
+  else if (n <= 16)
     launch_zgemm_dmma<64, 16, 16, 16, 8, 3>(h, g, batch);
   else if (m <= 32)
     launch_zgemm_dmma<32, 64, 32, 16, 8, 3>(h, g, batch);
+  else if (k <= 64 && tall && n > 32)
+    launch_zgemm_dmma<64, 64, 32, 16, 8, 3>(h, g, batch);
   else if (k <= 64)
     launch_zgemm_dmma<32, 32, 16, 16, 8, 3>(h, g, batch);
   else if (m <= 64 && n >= 128)
