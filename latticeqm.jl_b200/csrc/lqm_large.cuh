@@ -1241,7 +1241,9 @@ __global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, doubl
   extern __shared__ __align__(16) double2 tswin[];
   __shared__ long long prog[kTsPairs];
   __shared__ int stop;
-  __shared__ int halt[kTsPairs];  // the maker gave up (read by the applier after their barrier)
+  // the meeting at which the maker gives up, or -1: a number, as the applier may still be on its
+  // way from the last meeting when the maker writes it, and has to come to this one too
+  __shared__ int halt[kTsPairs];
   constexpr int B = kTsB, LW = kTsLw, ldb = 2 * B;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, pair = w >> 1;
   const bool maker = (w & 1) == 0;
@@ -1255,7 +1257,7 @@ __global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, doubl
   double2* sc = wv + B;                      // tau, (beta, 0) of even and odd tasks
   const int tmax = ts_tmax(n, B);
   const long long unit = tmax + 1;  // progress: s * unit + tasks done
-  if (threadIdx.x < kTsPairs) { prog[threadIdx.x] = -1; halt[threadIdx.x] = 0; }
+  if (threadIdx.x < kTsPairs) { prog[threadIdx.x] = -1; halt[threadIdx.x] = -1; }
   if (threadIdx.x == 0) stop = (err && *(volatile int*)err) ? 1 : 0;
   __syncthreads();
   volatile long long* vprog = prog;
@@ -1334,14 +1336,14 @@ __global__ void __launch_bounds__(kTsPairs * 64, 1) ts_chase_kernel(int n, doubl
         meet();  // v, E and the reflector's scalars are the applier's; it is done with task t - 1
       }
       if (!ok) {
-        if (lane == 0) halt[pair] = 1;
+        if (lane == 0) ((volatile int*)halt)[pair] = it;
         meet();
         break;
       }
     } else {
       for (int t = 0; t < nt; ++t, ++it) {
         meet();
-        if (((volatile int*)halt)[pair]) { ok = false; break; }
+        if (((volatile int*)halt)[pair] == it) { ok = false; break; }
         const int R0 = s + 1 + t * B, c = t == 0 ? s : R0 - B;
         double2 D[8];  // D(r, 8 hh + k), the lower triangle
 #pragma unroll

@@ -546,7 +546,7 @@ static int emul_chase_pairs(int n, const double* band, int pairs, unsigned seed,
   struct Pair {
     double2 blk[3][B * LW], v[2][B], tau[2], beta[2];
     std::atomic<int> arrived{0}, turn{0};
-    int halt = 0;
+    std::atomic<int> halt{-1};
     void meet() {
       const int mine = turn.load(std::memory_order_acquire);
       if (arrived.fetch_add(1, std::memory_order_acq_rel) == 1) {
@@ -584,7 +584,7 @@ static int emul_chase_pairs(int n, const double* band, int pairs, unsigned seed,
           }
         }
         if (!ok) {
-          q.halt = 1;
+          q.halt.store(it, std::memory_order_relaxed);
           q.meet();
           return;
         }
@@ -624,7 +624,7 @@ static int emul_chase_pairs(int n, const double* band, int pairs, unsigned seed,
       const int nt = ts_tasks(n, B, s);
       for (int t = 0; t < nt; ++t, ++it) {
         q.meet();
-        if (q.halt) return;
+        if (q.halt.load(std::memory_order_relaxed) == it) return;
         rest(rng);
         const int R0 = s + 1 + t * B, c = t == 0 ? s : R0 - B, L = std::min(B, n - R0);
         double2* X = q.blk[it % 3];

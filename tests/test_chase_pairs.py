@@ -34,6 +34,7 @@ def test_pairs_match_the_sequential_chase(emul, b, n):
 
 
 def test_a_wait_that_expires_ends_every_pair(emul):
-    """A limit of one poll: whichever waits run out, all workers return (else the test hangs)."""
-    ended = [chase(emul, 131, 16, 8, seed, limit=1) for seed in range(6)]
+    """A limit of a few polls: whichever waits run out, all workers return (else the test hangs:
+    an applier still on its way from the last meeting has to come to the maker's final one)."""
+    ended = [chase(emul, 131, 16, 8, seed, limit=1 + seed % 3) for seed in range(600)]
     assert set(ended) <= {1, 2} and 2 in ended
